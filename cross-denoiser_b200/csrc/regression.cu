@@ -10,6 +10,7 @@
 // Coefficient layout in the workspace: beta[buf][b][j][i][r][ch] with
 // r = 0..5 the regression coefficient (constant, colour, albedo, normal.xyz)
 // and ch = 0..2 the colour channel; 18 floats per centre and buffer.
+#include <type_traits>
 #include <cuda_runtime.h>
 #include "cd_common.cuh"
 #include "f32x2.cuh"
@@ -160,29 +161,31 @@ __global__ void __launch_bounds__(256) variance_px_kernel(const float *__restric
 //   shared (10): A00 A03 A04 A05 A33 A34 A35 A44 A45 A55
 //   per channel (11 x 3): A01 A02 A11 A12 A13 A14 A15 A22 A23 A24 A25
 //   right-hand side (6 x 3): X0..X5
-// The per-channel terms of channels 0 and 1 are packed FP32x2 pairs (low
-// lane channel 0) updated by one fma.rn.f32x2 each, channel 2 stays scalar:
-// every lane is rounded as the scalar update, in the same order.
+// 58 of them are kept as packed FP32x2 pairs updated by one fma.rn.f32x2
+// each, every lane rounded as the scalar update and in the same order:
+// channels 0 and 1 side by side (p, px; low lane channel 0), and the shared
+// terms with channel 2's (q, x) so that the two lanes share one factor (w,
+// w dn_i, w d1 or w da) and the other is a pair at hand, (dn0, dn1), (dn2, y)
+// or (d1, da).  a05x0 = (A05, channel 2's X0), and so on.
 // ---------------------------------------------------------------------------
 struct Normal {
-    float a00, a03, a04, a05, a33, a34, a35, a44, a45, a55;
+    float a00, a44, q22;
+    x2::f2 a03a04, a05x0, a33a34, a35x3, a45x4, a55x5, q01q02, q11q12, q13q14, q15x1, q23q24, q25x2;
     x2::f2 p01, p02, p11, p12, p13, p14, p15, p22, p23, p24, p25;   // channels 0, 1
     x2::f2 px0, px1, px2, px3, px4, px5;
-    float q01, q02, q11, q12, q13, q14, q15, q22, q23, q24, q25;      // channel 2
-    float qx0, qx1, qx2, qx3, qx4, qx5;
 };
 
 CD_DEV void normal_zero(Normal &n)
 {
-    n.a00 = n.a03 = n.a04 = n.a05 = n.a33 = n.a34 = n.a35 = n.a44 = n.a45 = n.a55 = 0.f;
-    const x2::f2 z = x2::pack(0.f, 0.f);
+    n.a00 = n.a44 = n.q22 = 0.f;
+    const x2::f2 z = 0ull;   // +0.0f in both lanes
+    n.a03a04 = n.a05x0 = n.a33a34 = n.a35x3 = n.a45x4 = n.a55x5 = z;
+    n.q01q02 = n.q11q12 = n.q13q14 = n.q15x1 = n.q23q24 = n.q25x2 = z;
     n.p01 = n.p02 = n.p11 = n.p12 = n.p13 = n.p14 = n.p15 = n.p22 = n.p23 = n.p24 = n.p25 = z;
     n.px0 = n.px1 = n.px2 = n.px3 = n.px4 = n.px5 = z;
-    n.q01 = n.q02 = n.q11 = n.q12 = n.q13 = n.q14 = n.q15 = n.q22 = n.q23 = n.q24 = n.q25 = 0.f;
-    n.qx0 = n.qx1 = n.qx2 = n.qx3 = n.qx4 = n.qx5 = 0.f;
 }
 
-// channel k (0, 1: a lane of the pair; 2: the scalar) of a per-channel term
+// channel k (0, 1: a lane of the pair; 2: q) of a per-channel term
 CD_DEV float chan(x2::f2 p, float q, int k) { return k == 0 ? x2::lo(p) : k == 1 ? x2::hi(p) : q; }
 
 // |v|^2 as the reference's compiled norm2 rounds it: fma(z, z, fma(x, x, y*y))
@@ -190,71 +193,122 @@ CD_DEV float chan(x2::f2 p, float q, int k) { return k == 0 ? x2::lo(p) : k == 1
 // x*x + y*y + z*z, see reproject.cu).
 CD_DEV float sqnorm(float x, float y, float z) { return fmaf(z, z, fmaf(x, x, y * y)); }
 
-// One window tap of one buffer: features f (centre fc), target y, variance
-// and standard deviation (v, sd), shared albedo / normal differences.
+// exp(x) = 2^(x log2 e) on the ex2.approx.ftz instruction (subnormal results
+// flushed to zero).
+CD_DEV float exp_ftz(float x)
+{
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.44269504088896341f));
+    return y;
+}
+
+// Quotients by a shared divisor (P. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34,
+// 1990): with y the reciprocal of b rounded to nearest, q = RN(a y) and the
+// exact residual r = a - q b, RN(q + r y) is the IEEE quotient a / b.  y is
+// the hardware approximation (1 ulp) after one Newton step, which differs
+// from the rounded reciprocal only within about 2^-46 of a rounding
+// boundary.  Valid while a, b, y and a / b stay away from the range's ends.
+CD_DEV float reciprocal(float b)
+{
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return fmaf(y, fmaf(-b, y, 1.f), y);
+}
+CD_DEV float quotient(float a, float b, float y)
+{
+    const float q = __fmul_rn(a, y);
+    return fmaf(fmaf(-q, b, a), y, q);
+}
+constexpr float kQuotientMax = 0x1p100f;
+
+// The centre's own values: features, albedo and normal (channels 0, 1 as a
+// pair), variance and standard deviation.
+struct Centre {
+    x2::f2 f01, a01, n01;
+    float f2, a2, n2, v, sd;
+};
+
+// One window tap of one buffer: f4 = (features, variance), y4 = (target, .),
+// a4 = (albedo, .), n4 = (normal, .), sdt the features' standard deviation.
 // Follows ops/regression.cu.cc:418-445: delta = [1, (f_t-f_c)/(sd_c+sd_t+1e-2),
 // alb_t-alb_c, n_t-n_c], w = exp(-|f_t-f_c|^2/(v_c+v_t+1e-4)) + 1e-7.
-CD_DEV void normal_tap(Normal &n, float3 ft, float3 fc, float3 y, float vt, float vc, float sdt,
-                       float sdc, const float da[3], const float dn[3])
+//
+// The tap's four quotients are the IEEE quotients: the normal equations
+// amplify their last bits.  kFast takes them with quotient() from two
+// reciprocals instead of four divisions (about 20 instructions each, with a
+// branch): 1080p, window 17, the kernel 505 -> 433 us (and 407 us with the
+// pairs, the fixed row layout and the launch bound below).  That needs the
+// divisors (at least 1e-4) and the squared distance below kQuotientMax,
+// which bounds the other operands too (sd = sqrt(v)); `sane` turns false
+// where a tap is not, and the caller repeats its window with kFast off.
+template <bool kFast>
+CD_DEV void normal_tap(Normal &n, float4 f4, float4 y4, float4 a4, float4 n4, float sdt, const Centre &c, bool &sane)
 {
     using namespace x2;
-    const float df[3] = {ft.x - fc.x, ft.y - fc.y, ft.z - fc.z};
-    const float den = (sdc + sdt) + 1e-2f;
-    const float dist = sqnorm(df[0], df[1], df[2]) / ((vc + vt) + 1e-4f);
-    const float w = __expf(-dist) + 1e-7f;
-    const float wn0 = w * dn[0], wn1 = w * dn[1], wn2 = w * dn[2];
-    n.a00 += w;
-    n.a03 = fmaf(w, dn[0], n.a03);
-    n.a04 = fmaf(w, dn[1], n.a04);
-    n.a05 = fmaf(w, dn[2], n.a05);
-    n.a33 = fmaf(wn0, dn[0], n.a33);
-    n.a34 = fmaf(wn0, dn[1], n.a34);
-    n.a35 = fmaf(wn0, dn[2], n.a35);
-    n.a44 = fmaf(wn1, dn[1], n.a44);
-    n.a45 = fmaf(wn1, dn[2], n.a45);
-    n.a55 = fmaf(wn2, dn[2], n.a55);
-    // channels 0 and 1
-    const f2 wP = pack(w, w), d1P = pack(df[0] / den, df[1] / den), daP = pack(da[0], da[1]);
-    const f2 wd1P = mul2(wP, d1P), wd2P = mul2(wP, daP);
-    const f2 dn0P = pack(dn[0], dn[0]), dn1P = pack(dn[1], dn[1]), dn2P = pack(dn[2], dn[2]);
-    const f2 yP = pack(y.x, y.y);
+    const f2 df01 = sub2(pack(f4.x, f4.y), c.f01), da01 = sub2(pack(a4.x, a4.y), c.a01);
+    const f2 dn01 = sub2(pack(n4.x, n4.y), c.n01);
+    const float df2 = f4.z - c.f2, da2 = a4.z - c.a2, dn2 = n4.z - c.n2;
+    const float den = (c.sd + sdt) + 1e-2f;
+    const float denw = (c.v + f4.w) + 1e-4f, sq = sqnorm(lo(df01), hi(df01), df2);
+    float dist, d1[3];
+    if (kFast) {
+        sane = sane && denw < kQuotientMax && sq < kQuotientMax;
+        const float rden = reciprocal(den), rw = reciprocal(denw);
+        dist = quotient(sq, denw, rw);
+        d1[0] = quotient(lo(df01), den, rden);
+        d1[1] = quotient(hi(df01), den, rden);
+        d1[2] = quotient(df2, den, rden);
+    } else {
+        dist = sq / denw;
+        d1[0] = lo(df01) / den;
+        d1[1] = hi(df01) / den;
+        d1[2] = df2 / den;
+    }
+    // a weight below 2^-126 and its flush to zero both give 1e-7 after the addition
+    const float w = exp_ftz(-dist) + 1e-7f;
+    const f2 wP = pack(w, w), d1P = pack(d1[0], d1[1]), yP = pack(y4.x, y4.y);
+    const f2 dda = pack(d1[2], da2), dny = pack(dn2, y4.z);   // channel 2's (d1, da) and (dn2, y)
+    const f2 wd1P = mul2(wP, d1P), wd2P = mul2(wP, da01), wdda = mul2(wP, dda), wn01 = mul2(wP, dn01);
+    const f2 dn0P = pack(lo(dn01), lo(dn01)), dn1P = pack(hi(dn01), hi(dn01)), dn2P = pack(dn2, dn2);
+    const f2 wn0P = pack(lo(wn01), lo(wn01)), wn1P = pack(hi(wn01), hi(wn01));
+    const float wn2 = w * dn2;
+    const f2 wn2P = pack(wn2, wn2);
     n.p01 = fma2(wP, d1P, n.p01);
-    n.p02 = fma2(wP, daP, n.p02);
+    n.p02 = fma2(wP, da01, n.p02);
     n.p11 = fma2(wd1P, d1P, n.p11);
-    n.p12 = fma2(wd1P, daP, n.p12);
+    n.p12 = fma2(wd1P, da01, n.p12);
     n.p13 = fma2(wd1P, dn0P, n.p13);
     n.p14 = fma2(wd1P, dn1P, n.p14);
     n.p15 = fma2(wd1P, dn2P, n.p15);
-    n.p22 = fma2(wd2P, daP, n.p22);
+    n.p22 = fma2(wd2P, da01, n.p22);
     n.p23 = fma2(wd2P, dn0P, n.p23);
     n.p24 = fma2(wd2P, dn1P, n.p24);
     n.p25 = fma2(wd2P, dn2P, n.p25);
     n.px0 = fma2(wP, yP, n.px0);
     n.px1 = fma2(wd1P, yP, n.px1);
     n.px2 = fma2(wd2P, yP, n.px2);
-    n.px3 = fma2(pack(wn0, wn0), yP, n.px3);
-    n.px4 = fma2(pack(wn1, wn1), yP, n.px4);
-    n.px5 = fma2(pack(wn2, wn2), yP, n.px5);
-    // channel 2
-    const float d1 = df[2] / den;
-    const float wd1 = w * d1, wd2 = w * da[2];
-    n.q01 = fmaf(w, d1, n.q01);
-    n.q02 = fmaf(w, da[2], n.q02);
-    n.q11 = fmaf(wd1, d1, n.q11);
-    n.q12 = fmaf(wd1, da[2], n.q12);
-    n.q13 = fmaf(wd1, dn[0], n.q13);
-    n.q14 = fmaf(wd1, dn[1], n.q14);
-    n.q15 = fmaf(wd1, dn[2], n.q15);
-    n.q22 = fmaf(wd2, da[2], n.q22);
-    n.q23 = fmaf(wd2, dn[0], n.q23);
-    n.q24 = fmaf(wd2, dn[1], n.q24);
-    n.q25 = fmaf(wd2, dn[2], n.q25);
-    n.qx0 = fmaf(w, y.z, n.qx0);
-    n.qx1 = fmaf(wd1, y.z, n.qx1);
-    n.qx2 = fmaf(wd2, y.z, n.qx2);
-    n.qx3 = fmaf(wn0, y.z, n.qx3);
-    n.qx4 = fmaf(wn1, y.z, n.qx4);
-    n.qx5 = fmaf(wn2, y.z, n.qx5);
+    n.px3 = fma2(wn0P, yP, n.px3);
+    n.px4 = fma2(wn1P, yP, n.px4);
+    n.px5 = fma2(wn2P, yP, n.px5);
+    // shared terms and channel 2
+    const float wd1 = lo(wdda), wd2 = hi(wdda);
+    const f2 wd1D = pack(wd1, wd1), wd2D = pack(wd2, wd2);
+    n.a00 += w;
+    n.a44 = fmaf(hi(wn01), hi(dn01), n.a44);
+    n.q22 = fmaf(wd2, da2, n.q22);
+    n.a03a04 = fma2(wP, dn01, n.a03a04);
+    n.a05x0 = fma2(wP, dny, n.a05x0);
+    n.a33a34 = fma2(wn0P, dn01, n.a33a34);
+    n.a35x3 = fma2(wn0P, dny, n.a35x3);
+    n.a45x4 = fma2(wn1P, dny, n.a45x4);
+    n.a55x5 = fma2(wn2P, dny, n.a55x5);
+    n.q01q02 = fma2(wP, dda, n.q01q02);
+    n.q11q12 = fma2(wd1D, dda, n.q11q12);
+    n.q13q14 = fma2(wd1D, dn01, n.q13q14);
+    n.q15x1 = fma2(wd1D, dny, n.q15x1);
+    n.q23q24 = fma2(wd2D, dn01, n.q23q24);
+    n.q25x2 = fma2(wd2D, dny, n.q25x2);
 }
 
 // Cholesky factorisation + forward / backward substitution of one channel's
@@ -308,19 +362,22 @@ CD_DEV void solve_channel(const Normal &n, int k, float *beta, float *Lo, float 
                           unsigned *fallbacks = nullptr)
 {
     float A[kP][kP];
-    A[0][0] = n.a00; A[0][1] = chan(n.p01, n.q01, k); A[0][2] = chan(n.p02, n.q02, k);
-    A[0][3] = n.a03; A[0][4] = n.a04; A[0][5] = n.a05;
-    A[1][1] = chan(n.p11, n.q11, k); A[1][2] = chan(n.p12, n.q12, k); A[1][3] = chan(n.p13, n.q13, k);
-    A[1][4] = chan(n.p14, n.q14, k); A[1][5] = chan(n.p15, n.q15, k);
-    A[2][2] = chan(n.p22, n.q22, k); A[2][3] = chan(n.p23, n.q23, k); A[2][4] = chan(n.p24, n.q24, k);
-    A[2][5] = chan(n.p25, n.q25, k);
-    A[3][3] = n.a33; A[3][4] = n.a34; A[3][5] = n.a35;
-    A[4][4] = n.a44; A[4][5] = n.a45;
-    A[5][5] = n.a55;
+    using x2::lo;
+    using x2::hi;
+    A[0][0] = n.a00; A[0][1] = chan(n.p01, lo(n.q01q02), k); A[0][2] = chan(n.p02, hi(n.q01q02), k);
+    A[0][3] = lo(n.a03a04); A[0][4] = hi(n.a03a04); A[0][5] = lo(n.a05x0);
+    A[1][1] = chan(n.p11, lo(n.q11q12), k); A[1][2] = chan(n.p12, hi(n.q11q12), k);
+    A[1][3] = chan(n.p13, lo(n.q13q14), k); A[1][4] = chan(n.p14, hi(n.q13q14), k);
+    A[1][5] = chan(n.p15, lo(n.q15x1), k);
+    A[2][2] = chan(n.p22, n.q22, k); A[2][3] = chan(n.p23, lo(n.q23q24), k);
+    A[2][4] = chan(n.p24, hi(n.q23q24), k); A[2][5] = chan(n.p25, lo(n.q25x2), k);
+    A[3][3] = lo(n.a33a34); A[3][4] = hi(n.a33a34); A[3][5] = lo(n.a35x3);
+    A[4][4] = n.a44; A[4][5] = lo(n.a45x4);
+    A[5][5] = lo(n.a55x5);
 #pragma unroll
     for (int r = 0; r < kP; ++r) A[r][r] += 1e-3f;
-    const float X[kP] = {chan(n.px0, n.qx0, k), chan(n.px1, n.qx1, k), chan(n.px2, n.qx2, k),
-                         chan(n.px3, n.qx3, k), chan(n.px4, n.qx4, k), chan(n.px5, n.qx5, k)};
+    const float X[kP] = {chan(n.px0, hi(n.a05x0), k), chan(n.px1, hi(n.q15x1), k), chan(n.px2, hi(n.q25x2), k),
+                         chan(n.px3, hi(n.a35x3), k), chan(n.px4, hi(n.a45x4), k), chan(n.px5, hi(n.a55x5), k)};
     float L[kP][kP];
 #pragma unroll
     for (int i = 0; i < kP; ++i) {
@@ -390,33 +447,49 @@ constexpr int kCX = kRowCentres;   // centres per CTA
 constexpr int kThreads = 64;
 
 // two row slots of 4 float4 groups, then the per-position tables
-__host__ __device__ inline size_t regression_smem(int hw, int sp)
+//
+// SP > 0: the sparsity as a template parameter, and a fixed row layout
+// (row_q(SP) positions per de-interleaved run, enough for windows to 19), so
+// that a tap's four loads and the SP taps of a run are constant offsets from
+// one pointer.  SP = 4, the reference's, and 2; others take SP = 0.  The
+// positions are no more than the windows need: a longer run measured slower
+// (40 instead of 36 at SP = 4: 713 against 706 us per 1080p
+// cross-regression, window 17), shared memory being taken from the L1 that
+// the neighbouring CTAs' rows hit.
+__host__ __device__ constexpr int row_q(int sp) { return kCX - 1 + (19 + sp - 1) / sp; }
+
+template <int SP>
+__host__ __device__ inline RowGeom regression_geom(int hw, int sp)
 {
-    const RowGeom g = row_geom(hw, sp);
+    RowGeom g = row_geom(hw, sp);
+    if (SP > 0) {
+        g.q = row_q(SP);
+        g.npos = SP * g.q;
+    }
+    return g;
+}
+
+inline bool fixed_rows(int hw, int sp) { return (sp == 2 || sp == 4) && row_geom(hw, sp).q <= row_q(sp); }
+
+__host__ __device__ inline size_t regression_smem(const RowGeom &g)
+{
     return (size_t)2 * 4 * g.npos * sizeof(float4) + (size_t)2 * g.rw * sizeof(int);
 }
 
-// exp(x) = 2^(x log2 e) on the ex2.approx.ftz instruction (subnormal results
-// flushed to zero).
-CD_DEV float exp_ftz(float x)
-{
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x * 1.44269504088896341f));
-    return y;
-}
-
-// Launch bound 7 CTAs per SM: the compiler still fits 128 registers (8 CTAs
-// per SM reside) and schedules the one-time solve with fewer spills than
-// under a bound of 8 (603 against 613 us per 1920x1080 cross-regression).
-__global__ void __launch_bounds__(kThreads, 7) regression_kernel(
+// Launch bound 8 CTAs per SM (128 registers): 706 us per 1080p
+// cross-regression, window 17, against 733 under a bound of 7, 776 under 6
+// (154 registers, 12 warps per SM) and 757 under 9 (112, spills in the sums).
+template <int SP>
+__global__ void __launch_bounds__(kThreads, 8) regression_kernel(
     const float *__restrict__ imga, const float *__restrict__ imgb,
     const float *__restrict__ albedo, const float *__restrict__ normal,
     const float *__restrict__ vara, const float *__restrict__ varb,
     const float *__restrict__ sda, const float *__restrict__ sdb, float *__restrict__ beta,
-    float *__restrict__ chol, float cond_limit, unsigned *__restrict__ fallbacks, int H, int W, int hw, int sp)
+    float *__restrict__ chol, float cond_limit, unsigned *__restrict__ fallbacks, int H, int W, int hw, int sp_rt)
 {
     extern __shared__ float4 sm4[];
-    const RowGeom g = row_geom(hw, sp);
+    const int sp = SP > 0 ? SP : sp_rt;
+    const RowGeom g = regression_geom<SP>(hw, sp);
     const int slot = 4 * g.npos;                                   // float4s per slot
     int *pos_gx = reinterpret_cast<int *>(sm4 + 2 * slot);
     int *pos_dst = pos_gx + g.rw;
@@ -448,50 +521,62 @@ __global__ void __launch_bounds__(kThreads, 7) regression_kernel(
                          sdb, threadIdx.x, kThreads);
     };
 
-    stage(0, 0);
-    cp_async_commit();
-
     // centre values, read directly (clamped for lanes past the last centre)
     const int ci = min(i0 + lane, Ws - 1);
     const size_t c = (size_t)cy * W + (size_t)ci * sp;
     const float3 fc = ld3(buf ? imgb : imga, c);
     const float3 alc = ld3(albedo, c), nrc = ld3(normal, c);
     const float vc = __ldg((buf ? varb : vara) + c), sdc = __ldg((buf ? sdb : sda) + c);
-    const float al_c[3] = {alc.x, alc.y, alc.z}, nr_c[3] = {nrc.x, nrc.y, nrc.z};
+    const Centre cen = {x2::pack(fc.x, fc.y), x2::pack(alc.x, alc.y), x2::pack(nrc.x, nrc.y), fc.z, alc.z, nrc.z,
+                        vc, sdc};
     // groups read by this buffer: own features + variance, target, albedo, normal
     const int gf = buf ? 1 : 0, gy_ = buf ? 0 : 1;
 
     Normal nm;
-    normal_zero(nm);
-    for (int r = 0; r < R; ++r) {
-        if (r + 1 < R) {
-            stage(r + 1, (r + 1) & 1);
-            cp_async_commit();
-            cp_async_wait<1>();
-        } else {
-            cp_async_wait<0>();
-        }
-        __syncthreads();
-        const float4 *P = sm4 + (r & 1) * slot;
-        const float4 *Gf = P + gf * g.npos, *Gy = P + gy_ * g.npos;
-        const float4 *Ga = P + 2 * g.npos, *Gn = P + 3 * g.npos;
-        int tm = 0, td = 0;
-        for (int t = 0; t < R; ++t) {
-            const int o = tm * g.q + td + lane;
-            const float4 f4 = Gf[o], y4 = Gy[o], a4 = Ga[o], n4 = Gn[o];
-            // own standard deviation: sdA rides in g2.w, sdB in g3.w
-            const float sdt = buf ? n4.w : a4.w;
-            const float da[3] = {a4.x - al_c[0], a4.y - al_c[1], a4.z - al_c[2]};
-            const float dn[3] = {n4.x - nr_c[0], n4.y - nr_c[1], n4.z - nr_c[2]};
-            normal_tap(nm, make_float3(f4.x, f4.y, f4.z), fc, make_float3(y4.x, y4.y, y4.z), f4.w, vc, sdt,
-                       sdc, da, dn);
-            if (++tm == sp) {
-                tm = 0;
-                ++td;
+    // the sum over the window's taps; whether every quotient was in range
+    auto sweep = [&](auto fast) {
+        bool sane = true;
+        normal_zero(nm);
+        stage(0, 0);
+        cp_async_commit();
+        for (int r = 0; r < R; ++r) {
+            if (r + 1 < R) {
+                stage(r + 1, (r + 1) & 1);
+                cp_async_commit();
+                cp_async_wait<1>();
+            } else {
+                cp_async_wait<0>();
             }
+            __syncthreads();
+            const float4 *P = sm4 + (r & 1) * slot;
+            const float4 *Gf = P + gf * g.npos + lane, *Gy = P + gy_ * g.npos + lane;
+            const float4 *Gn = P + 3 * g.npos + lane;   // albedo: g.npos before it
+            auto tap = [&](int o) {
+                const float4 f4 = Gf[o], y4 = Gy[o], a4 = Gn[o - g.npos], n4 = Gn[o];
+                // own standard deviation: sdA rides in g2.w, sdB in g3.w
+                normal_tap<decltype(fast)::value>(nm, f4, y4, a4, n4, buf ? n4.w : a4.w, cen, sane);
+            };
+            if (SP > 0) {
+                for (int t = 0; t < R; t += sp, ++Gf, ++Gy, ++Gn) {
+#pragma unroll
+                    for (int tm = 0; tm < SP; ++tm)
+                        if (t + tm < R) tap(tm * g.q);
+                }
+            } else {
+                int tm = 0, td = 0;
+                for (int t = 0; t < R; ++t) {
+                    tap(tm * g.q + td);
+                    if (++tm == sp) {
+                        tm = 0;
+                        ++td;
+                    }
+                }
+            }
+            __syncthreads();
         }
-        __syncthreads();
-    }
+        return sane;
+    };
+    if (!__syncthreads_and(sweep(std::true_type()))) sweep(std::false_type());
 
     if (i0 + lane >= Ws) return;
     const size_t nb_img = (size_t)Hs * Ws;
@@ -679,7 +764,7 @@ cudaError_t launch_variance(const float *imga, const float *imgb, float *vara, f
     return cudaGetLastError();
 }
 
-size_t regression_smem_bytes(int win, int sp) { return regression_smem(win / 2, sp); }
+size_t regression_smem_bytes(int win, int sp) { return regression_smem(row_geom(win / 2, sp)); }
 size_t recon_smem_bytes(int win, int sp, int rs) { return recon_smem(win / 2, sp, rs); }
 
 cudaError_t launch_regression(const float *imga, const float *imgb, const float *albedo,
@@ -689,15 +774,19 @@ cudaError_t launch_regression(const float *imga, const float *imgb, const float 
                               unsigned *fallbacks)
 {
     const int hw = win / 2;
-    const size_t smem = regression_smem(hw, sp);
-    cudaError_t e = cudaFuncSetAttribute(regression_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
     const int Ws = W / sp, Hs = H / sp;
     dim3 grid((Ws + kCX - 1) / kCX, Hs, B);
-    regression_kernel<<<grid, kThreads, smem, st>>>(imga, imgb, albedo, normal, vara, varb, sda, sdb, beta,
-                                                    chol, cond_limit, fallbacks, H, W, hw, sp);
-    return cudaGetLastError();
+    auto go = [&](auto kern, const RowGeom &g) {
+        const size_t smem = regression_smem(g);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        kern<<<grid, kThreads, smem, st>>>(imga, imgb, albedo, normal, vara, varb, sda, sdb, beta, chol, cond_limit,
+                                           fallbacks, H, W, hw, sp);
+        return cudaGetLastError();
+    };
+    if (!fixed_rows(hw, sp)) return go(regression_kernel<0>, regression_geom<0>(hw, sp));
+    return sp == 4 ? go(regression_kernel<4>, regression_geom<4>(hw, sp))
+                   : go(regression_kernel<2>, regression_geom<2>(hw, sp));
 }
 
 cudaError_t launch_recon(const float *imga, const float *imgb, const float *albedo,
