@@ -605,19 +605,38 @@ __global__ void __launch_bounds__(kThreads, 8) regression_kernel(
 //   9      (feature.x, feature.y)      10  (feature.z, variance)
 //   11     (sd, albedo.x albedo.y)     12  albedo.z normal.xyz (scalars)
 // ---------------------------------------------------------------------------
-constexpr int kRX = 32, kRY = 4;
+constexpr int kRX = 32, kRThreadRows = 4;
 constexpr int kRec = 13;   // float4 per staged centre
+
+// Two pixels per thread while three CTAs' centres fit an SM's shared
+// memory, one for the wider windows and denser centres.
+constexpr size_t kReconPairSmem = 74 * 1024;
 
 __host__ __device__ inline int floordiv(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
-__host__ __device__ inline size_t recon_smem(int hw, int sp, int rs)
+__host__ __device__ inline size_t recon_smem(int hw, int sp, int rs, int rows)
 {
     const int cxmax = ((kRX - 1) * rs + 2 * hw) / sp + 2;
-    const int cymax = ((kRY - 1) * rs + 2 * hw) / sp + 2;
+    const int cymax = ((rows - 1) * rs + 2 * hw) / sp + 2;
     return (size_t)kRec * cxmax * cymax * sizeof(float4);
 }
 
-__global__ void __launch_bounds__(kRX * kRY) recon_kernel(
+// One output pixel's own values ((A, B) pairs, shared scalars) and its sums.
+struct ReconPixel {
+    x2::f2 f0, f1, f2, var, sd;
+    float3 al, nr;
+    x2::f2 o0, o1, o2, sw;
+};
+
+// NP: output pixels per thread, in consecutive rows.  A record is 208 bytes
+// per lane, and shared memory returns 128 bytes per cycle and SM whatever
+// the lanes share, so with one pixel per thread the kernel runs at that rate
+// (92 % of it, 52 cycles per warp and centre against 19 of packed
+// arithmetic); two pixels per thread read each record once for both.  The
+// rows of a warp's pixels are the same, so the centre rows that only one of
+// them reaches are a uniform branch.
+template <int NP>
+__global__ void __launch_bounds__(kRX * kRThreadRows, NP == 2 ? 4 : 1) recon_kernel(
     const float *__restrict__ imga, const float *__restrict__ imgb,
     const float *__restrict__ albedo, const float *__restrict__ normal,
     const float *__restrict__ vara, const float *__restrict__ varb,
@@ -627,6 +646,7 @@ __global__ void __launch_bounds__(kRX * kRY) recon_kernel(
 {
     using namespace x2;
     extern __shared__ float4 rec[];
+    constexpr int kRows = NP * kRThreadRows, kBlock = kRX * kRThreadRows;
     const int Wr = W / rs, Hr = H / rs;
     const int Ws = W / sp, Hs = H / sp;
     const int b = blockIdx.z;
@@ -645,8 +665,8 @@ __global__ void __launch_bounds__(kRX * kRY) recon_kernel(
 
     // centres any pixel of this tile can reach (a superset of every
     // per-pixel range below)
-    const int ox0 = blockIdx.x * kRX, oy0 = blockIdx.y * kRY;
-    const int ox1 = min(ox0 + kRX - 1, Wr - 1), oy1 = min(oy0 + kRY - 1, Hr - 1);
+    const int ox0 = blockIdx.x * kRX, oy0 = blockIdx.y * kRows;
+    const int ox1 = min(ox0 + kRX - 1, Wr - 1), oy1 = min(oy0 + kRows - 1, Hr - 1);
     const int cx_lo = max(0, floordiv(ox0 * rs - hw, sp));
     const int cx_hi = min(Ws - 1, (ox1 * rs + hw) / sp);
     const int cy_lo = max(0, floordiv(oy0 * rs - hw, sp));
@@ -655,13 +675,13 @@ __global__ void __launch_bounds__(kRX * kRY) recon_kernel(
     const int nc = ncx * ncy;
 
     const int tid = threadIdx.y * kRX + threadIdx.x;
-    for (int e = tid; e < nc * 9; e += kRX * kRY) {
+    for (int e = tid; e < nc * 9; e += kBlock) {
         const int n = e / 9, f = e - 9 * n;
         const int iy = cy_lo + n / ncx, ix = cx_lo + n % ncx;
         const size_t cb = ((size_t)iy * Ws + ix) * kBeta + 2 * f;
         rec[n * kRec + f] = make_float4(__ldg(betaA + cb), __ldg(betaB + cb), __ldg(betaA + cb + 1), __ldg(betaB + cb + 1));
     }
-    for (int n = tid; n < nc; n += kRX * kRY) {
+    for (int n = tid; n < nc; n += kBlock) {
         const int iy = cy_lo + n / ncx, ix = cx_lo + n % ncx;
         const size_t t = (size_t)(iy * sp) * W + ix * sp;
         const float3 fa = ld3(imga, t), fb = ld3(imgb, t), al = ld3(albedo, t), nr = ld3(normal, t);
@@ -672,78 +692,120 @@ __global__ void __launch_bounds__(kRX * kRY) recon_kernel(
     }
     __syncthreads();
 
-    const int cx = ox0 + threadIdx.x, cy = oy0 + threadIdx.y;
+    const int cx = ox0 + threadIdx.x, cy = oy0 + NP * threadIdx.y;
     if (cx >= Wr || cy >= Hr) return;
-    const int pxo = cx * rs, pyo = cy * rs;
-    const size_t p = (size_t)pyo * W + pxo;
+    const int pxo = cx * rs;
     const int sx = max(0, idivup(pxo - hw, sp));
     const int ex = min((W - 1) / sp, (pxo + hw) / sp);
-    const int sy = max(0, idivup(pyo - hw, sp));
-    const int ey = min((H - 1) / sp, (pyo + hw) / sp);
-
-    const float3 fa = ld3(imga, p), fb = ld3(imgb, p), al = ld3(albedo, p), nr = ld3(normal, p);
-    const f2 pf_x = pack(fa.x, fb.x), pf_y = pack(fa.y, fb.y), pf_z = pack(fa.z, fb.z);
-    const f2 pvar = pack(__ldg(vara + p), __ldg(varb + p)), psd = pack(__ldg(sda + p), __ldg(sdb + p));
+    int sy[NP], ey[NP];
+    ReconPixel px_[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        const bool in = cy + i < Hr;
+        const int pyo = (in ? cy + i : cy) * rs;
+        const size_t p = (size_t)pyo * W + pxo;
+        sy[i] = max(0, idivup(pyo - hw, sp));
+        ey[i] = in ? min((H - 1) / sp, (pyo + hw) / sp) : -1;   // no centre row for a pixel past the image
+        const float3 fa = ld3(imga, p), fb = ld3(imgb, p);
+        ReconPixel &q = px_[i];
+        q.al = ld3(albedo, p);
+        q.nr = ld3(normal, p);
+        q.f0 = pack(fa.x, fb.x);
+        q.f1 = pack(fa.y, fb.y);
+        q.f2 = pack(fa.z, fb.z);
+        q.var = pack(__ldg(vara + p), __ldg(varb + p));
+        q.sd = pack(__ldg(sda + p), __ldg(sdb + p));
+        q.o0 = q.o1 = q.o2 = q.sw = 0ull;   // +0.0f in both lanes
+    }
     const f2 k1e2 = pack(1e-2f, 1e-2f), k1e4 = pack(1e-4f, 1e-4f), k1e7 = pack(1e-7f, 1e-7f);
-    f2 o0 = 0ull, o1 = 0ull, o2 = 0ull, sw = 0ull;   // +0.0f in both lanes
-    for (int iy = sy; iy <= ey; ++iy) {
-        const int nrow = (iy - cy_lo) * ncx - cx_lo;
-        for (int ix = sx; ix <= ex; ++ix) {
-            const float4 *R4 = rec + (nrow + ix) * kRec;
+    // the centres of row iy, for the pixels [i0, i0 + n)
+    auto centre_row = [&](int iy, auto first, auto count) {
+        constexpr int i0 = decltype(first)::value, n = decltype(count)::value;
+        const float4 *R4 = rec + ((iy - cy_lo) * ncx - cx_lo + sx) * kRec;
+        for (int ix = sx; ix <= ex; ++ix, R4 += kRec) {
             const ulonglong2 *R = reinterpret_cast<const ulonglong2 *>(R4);
             const ulonglong2 F9 = R[9], F10 = R[10], F11 = R[11];
             const float4 L12 = R4[12];
-            const float da0 = al.x - lo(F11.y), da1 = al.y - hi(F11.y), da2 = al.z - L12.x;
-            const float dn0 = nr.x - L12.y, dn1 = nr.y - L12.z, dn2 = nr.z - L12.w;
-            const f2 d0 = sub2(pf_x, F9.x), d1 = sub2(pf_y, F9.y), d2 = sub2(pf_z, F10.x);
-            const f2 den_r = add2(add2(psd, F11.x), k1e2);
-            const f2 rden = pack(__fdividef(1.f, lo(den_r)), __fdividef(1.f, hi(den_r)));
-            const f2 den_w = add2(add2(pvar, F10.y), k1e4);
-            const f2 q = mul2(sqnorm2(d0, d1, d2), pack(__fdividef(1.f, lo(den_w)), __fdividef(1.f, hi(den_w))));
-            // exp(-q) + 1e-7 with exp as 2^(-q log2 e) on ex2.approx.ftz: the
-            // same weight as __expf wherever exp(-q) is a normal float, and
-            // where it is not, both round to 1e-7 after the addition
-            const f2 w = add2(pack(exp_ftz(-lo(q)), exp_ftz(-hi(q))), k1e7);
-            const ulonglong2 c0 = R[0], c1 = R[1], c2 = R[2], c3 = R[3], c4 = R[4], c5 = R[5], c6 = R[6],
-                             c7 = R[7], c8 = R[8];
-            // coefficient j = r * 3 + ch sits in record j / 2, half j % 2:
-            // r 0: c0.x c0.y c1.x | r 1: c1.y c2.x c2.y | r 2: c3.x c3.y c4.x
-            // r 3: c4.y c5.x c5.y | r 4: c6.x c6.y c7.x | r 5: c7.y c8.x c8.y
-            f2 p0 = c0.x, p1 = c0.y, p2 = c1.x;
-            p0 = fma2(c1.y, mul2(d0, rden), p0);
-            p1 = fma2(c2.x, mul2(d1, rden), p1);
-            p2 = fma2(c2.y, mul2(d2, rden), p2);
-            p0 = fma2(c3.x, pack(da0, da0), p0);
-            p1 = fma2(c3.y, pack(da1, da1), p1);
-            p2 = fma2(c4.x, pack(da2, da2), p2);
-            const f2 n0 = pack(dn0, dn0), n1 = pack(dn1, dn1), n2 = pack(dn2, dn2);
-            p0 = fma2(c4.y, n0, p0);
-            p1 = fma2(c5.x, n0, p1);
-            p2 = fma2(c5.y, n0, p2);
-            p0 = fma2(c6.x, n1, p0);
-            p1 = fma2(c6.y, n1, p1);
-            p2 = fma2(c7.x, n1, p2);
-            p0 = fma2(c7.y, n2, p0);
-            p1 = fma2(c8.x, n2, p1);
-            p2 = fma2(c8.y, n2, p2);
-            o0 = fma2(w, p0, o0);
-            o1 = fma2(w, p1, o1);
-            o2 = fma2(w, p2, o2);
-            sw = add2(sw, w);
+            f2 e0[n], e1[n], e2[n], w[n];
+#pragma unroll
+            for (int i = 0; i < n; ++i) {
+                const ReconPixel &q = px_[i0 + i];
+                const f2 d0 = sub2(q.f0, F9.x), d1 = sub2(q.f1, F9.y), d2 = sub2(q.f2, F10.x);
+                const f2 den_r = add2(add2(q.sd, F11.x), k1e2);
+                const f2 rden = pack(__fdividef(1.f, lo(den_r)), __fdividef(1.f, hi(den_r)));
+                const f2 den_w = add2(add2(q.var, F10.y), k1e4);
+                const f2 dist =
+                    mul2(sqnorm2(d0, d1, d2), pack(__fdividef(1.f, lo(den_w)), __fdividef(1.f, hi(den_w))));
+                // exp(-dist) + 1e-7 with exp as 2^(-dist log2 e) on ex2.approx.ftz:
+                // the same weight as __expf wherever it is a normal float, and
+                // where it is not, both round to 1e-7 after the addition
+                w[i] = add2(pack(exp_ftz(-lo(dist)), exp_ftz(-hi(dist))), k1e7);
+                e0[i] = mul2(d0, rden);
+                e1[i] = mul2(d1, rden);
+                e2[i] = mul2(d2, rden);
+            }
+            const ulonglong2 c0 = R[0], c1 = R[1], c2 = R[2], c3 = R[3], c4 = R[4], c5 = R[5], c6 = R[6], c7 = R[7],
+                             c8 = R[8];
+#pragma unroll
+            for (int i = 0; i < n; ++i) {
+                ReconPixel &q = px_[i0 + i];
+                const float da0 = q.al.x - lo(F11.y), da1 = q.al.y - hi(F11.y), da2 = q.al.z - L12.x;
+                const float dn0 = q.nr.x - L12.y, dn1 = q.nr.y - L12.z, dn2 = q.nr.z - L12.w;
+                // coefficient j = r * 3 + ch sits in record j / 2, half j % 2:
+                // r 0: c0.x c0.y c1.x | r 1: c1.y c2.x c2.y | r 2: c3.x c3.y c4.x
+                // r 3: c4.y c5.x c5.y | r 4: c6.x c6.y c7.x | r 5: c7.y c8.x c8.y
+                f2 p0 = fma2(c1.y, e0[i], c0.x);
+                f2 p1 = fma2(c2.x, e1[i], c0.y);
+                f2 p2 = fma2(c2.y, e2[i], c1.x);
+                p0 = fma2(c3.x, pack(da0, da0), p0);
+                p1 = fma2(c3.y, pack(da1, da1), p1);
+                p2 = fma2(c4.x, pack(da2, da2), p2);
+                const f2 n0 = pack(dn0, dn0), n1 = pack(dn1, dn1), n2 = pack(dn2, dn2);
+                p0 = fma2(c4.y, n0, p0);
+                p1 = fma2(c5.x, n0, p1);
+                p2 = fma2(c5.y, n0, p2);
+                p0 = fma2(c6.x, n1, p0);
+                p1 = fma2(c6.y, n1, p1);
+                p2 = fma2(c7.x, n1, p2);
+                p0 = fma2(c7.y, n2, p0);
+                p1 = fma2(c8.x, n2, p1);
+                p2 = fma2(c8.y, n2, p2);
+                q.o0 = fma2(w[i], p0, q.o0);
+                q.o1 = fma2(w[i], p1, q.o1);
+                q.o2 = fma2(w[i], p2, q.o2);
+                q.sw = add2(q.sw, w[i]);
+            }
+        }
+    };
+    using std::integral_constant;
+    const int iy1 = NP == 2 ? max(ey[0], ey[NP - 1]) : ey[0];
+    for (int iy = NP == 2 ? min(sy[0], sy[NP - 1]) : sy[0]; iy <= iy1; ++iy) {
+        const bool in0 = iy >= sy[0] && iy <= ey[0], in1 = iy >= sy[NP - 1] && iy <= ey[NP - 1];
+        if (NP == 1 || !in1) {
+            if (in0) centre_row(iy, integral_constant<int, 0>(), integral_constant<int, 1>());
+        } else if (in0) {
+            centre_row(iy, integral_constant<int, 0>(), integral_constant<int, NP>());
+        } else {
+            centre_row(iy, integral_constant<int, NP - 1>(), integral_constant<int, 1>());
         }
     }
-    const float dA = fmaxf(lo(sw), 1e-7f), dB = fmaxf(hi(sw), 1e-7f);
-    const size_t o = (size_t)b * Hr * Wr + (size_t)cy * Wr + cx;
-    const float3 qa = make_float3(fmaxf(0.f, lo(o0) / dA), fmaxf(0.f, lo(o1) / dA), fmaxf(0.f, lo(o2) / dA));
-    const float3 qb = make_float3(fmaxf(0.f, hi(o0) / dB), fmaxf(0.f, hi(o1) / dB), fmaxf(0.f, hi(o2) / dB));
-    if (outa) {
-        st3(outa, o, qa);
-        st3(outb, o, qb);
-    }
-    if (state) {   // for the backward: the outputs and the weight sums D, [buffer][pixel]
-        float4 *S = reinterpret_cast<float4 *>(state);
-        S[o] = make_float4(qa.x, qa.y, qa.z, lo(sw));
-        S[(size_t)gridDim.z * Hr * Wr + o] = make_float4(qb.x, qb.y, qb.z, hi(sw));
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+        if (cy + i >= Hr) break;
+        const ReconPixel &q = px_[i];
+        const float dA = fmaxf(lo(q.sw), 1e-7f), dB = fmaxf(hi(q.sw), 1e-7f);
+        const size_t o = (size_t)b * Hr * Wr + (size_t)(cy + i) * Wr + cx;
+        const float3 qa = make_float3(fmaxf(0.f, lo(q.o0) / dA), fmaxf(0.f, lo(q.o1) / dA), fmaxf(0.f, lo(q.o2) / dA));
+        const float3 qb = make_float3(fmaxf(0.f, hi(q.o0) / dB), fmaxf(0.f, hi(q.o1) / dB), fmaxf(0.f, hi(q.o2) / dB));
+        if (outa) {
+            st3(outa, o, qa);
+            st3(outb, o, qb);
+        }
+        if (state) {   // for the backward: the outputs and the weight sums D, [buffer][pixel]
+            float4 *S = reinterpret_cast<float4 *>(state);
+            S[o] = make_float4(qa.x, qa.y, qa.z, lo(q.sw));
+            S[(size_t)gridDim.z * Hr * Wr + o] = make_float4(qb.x, qb.y, qb.z, hi(q.sw));
+        }
     }
 }
 
@@ -765,7 +827,7 @@ cudaError_t launch_variance(const float *imga, const float *imgb, float *vara, f
 }
 
 size_t regression_smem_bytes(int win, int sp) { return regression_smem(row_geom(win / 2, sp)); }
-size_t recon_smem_bytes(int win, int sp, int rs) { return recon_smem(win / 2, sp, rs); }
+size_t recon_smem_bytes(int win, int sp, int rs) { return recon_smem(win / 2, sp, rs, kRThreadRows); }
 
 cudaError_t launch_regression(const float *imga, const float *imgb, const float *albedo,
                               const float *normal, const float *vara, const float *varb,
@@ -795,16 +857,19 @@ cudaError_t launch_recon(const float *imga, const float *imgb, const float *albe
                          int W, int win, int sp, int rs, cudaStream_t st, float *state)
 {
     const int hw = win / 2;
-    const size_t smem = recon_smem(hw, sp, rs);
-    cudaError_t e = cudaFuncSetAttribute(recon_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
     const int Wr = W / rs, Hr = H / rs;
-    dim3 block(kRX, kRY);
-    dim3 grid((Wr + kRX - 1) / kRX, (Hr + kRY - 1) / kRY, B);
-    recon_kernel<<<grid, block, smem, st>>>(imga, imgb, albedo, normal, vara, varb, sda, sdb, beta, outa,
-                                            outb, state, H, W, hw, sp, rs);
-    return cudaGetLastError();
+    auto go = [&](auto kern, int np) {
+        const int rows = np * kRThreadRows;
+        const size_t smem = recon_smem(hw, sp, rs, rows);
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        dim3 block(kRX, kRThreadRows), grid((Wr + kRX - 1) / kRX, (Hr + rows - 1) / rows, B);
+        kern<<<grid, block, smem, st>>>(imga, imgb, albedo, normal, vara, varb, sda, sdb, beta, outa, outb, state, H,
+                                        W, hw, sp, rs);
+        return cudaGetLastError();
+    };
+    return recon_smem(hw, sp, rs, 2 * kRThreadRows) <= kReconPairSmem ? go(recon_kernel<2>, 2)
+                                                                      : go(recon_kernel<1>, 1);
 }
 
 }  // namespace cd
