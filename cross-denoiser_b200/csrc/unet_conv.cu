@@ -760,8 +760,9 @@ __global__ void __launch_bounds__(128) wgrad_kernel(const WgradParams P)
     if (warp == 0) tc::tmem_dealloc(tbase, kCols);
 }
 
-constexpr int kWgradThreads = 192;     // persistent weight gradient: producer, MMA, 4 bias warps
+constexpr int kWgradLoadWarps = 2;
 constexpr int kWgradBiasWarps = 4;
+constexpr int kWgradThreads = 32 * (kWgradLoadWarps + 1 + kWgradBiasWarps);   // producers, MMA, bias
 
 constexpr int kWgradRows = 4;
 
@@ -809,13 +810,16 @@ cudaError_t launch_wgrad_t(const WgradParams &P, int B, cudaStream_t st)
 // A tile is R input rows x 128 pixels: the output gradient's R + 2 rows from
 // y0 - 1 and the input rows, one bulk copy per plane with zeros outside the
 // image (stage_plane), land in a ring of S stages.  The warps specialise:
-// warp 0 stages tile i into slot i % S once the slot's "empty" barrier says
-// its previous MMAs and bias reads are done (all 32 lanes issue copies);
-// lane 0 of warp 1 issues the tile's MMAs when the slot is full and commits
-// them to "empty"; warps 2..5 sum the bias gradient (the output gradient
-// over the tile's R centre rows) from the staged planes and arrive on
-// "empty".  CTAs are persistent and keep their accumulators in TMEM over all
-// their tiles; one partial sum per CTA, read out of TMEM by warps 2..5 at
+// two producers stage tile i into slot i % S once the slot's "empty" barrier
+// says its previous MMAs and bias reads are done (all their lanes issue
+// copies; one producer issues a 2 KB copy about every 130-180 cycles, which
+// bounded the nine-tap form: 101 us with one, 82 with two, 80 with four for
+// 16 -> 8 channels at 2560x1440, a 1600 -> 1544 us training step);
+// a lane of the next warp issues the tile's MMAs when the slot is full and
+// commits them to "empty"; the last four warps sum the bias gradient (the
+// output gradient over the tile's R centre rows) from the staged planes and
+// arrive on "empty".  CTAs are persistent and keep their accumulators in TMEM over all
+// their tiles; one partial sum per CTA, read out of TMEM by the bias warps at
 // the end.  Every wait is bounded.
 constexpr int kWgrad3Smem = 225 * 1024;
 constexpr int kXPx = kPx + 2;                 // staged input pixels per row (three-tap form)
@@ -904,10 +908,10 @@ __global__ void __launch_bounds__(kWgradThreads, 1) wgrad3_kernel(const WgradPar
     uint32_t *tslot = reinterpret_cast<uint32_t *>(empty + S);
     float *red = reinterpret_cast<float *>(tail + 1024);   // [4][8 * ZC]
 
-    if (warp == 1) tc::tmem_alloc(tslot, cols);
+    if (warp == kWgradLoadWarps) tc::tmem_alloc(tslot, cols);
     if (tid == 0) {
         for (int s = 0; s < S; ++s) {
-            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&full[s], kWgradLoadWarps);
             tc::mbar_init(&empty[s], 1 + kWgradBiasWarps);   // the MMA commit + the bias warps
         }
         tc::fence_async_smem();
@@ -925,10 +929,13 @@ __global__ void __launch_bounds__(kWgradThreads, 1) wgrad3_kernel(const WgradPar
 #pragma unroll
     for (int j = 0; j < 8 * ZC; ++j) bsum[j] = 0.f;
 
-    if (warp == 0) {
-        // ---- producer: all lanes issue the planes of a stage ----
+    if (warp < kWgradLoadWarps) {
+        // ---- producers: all lanes issue the planes of a stage, producer w
+        // the planes w, w + kWgradLoadWarps, ... ----
         const int nz = (R + 2) * kZRow, nplanes = nz + R * xc;
-        const uint32_t tx_bytes = (uint32_t)(pl.zbytes + pl.xbytes);
+        const int my_z = (nz - warp + kWgradLoadWarps - 1) / kWgradLoadWarps;
+        const int my_all = (nplanes - warp + kWgradLoadWarps - 1) / kWgradLoadWarps;
+        const uint32_t tx_bytes = (uint32_t)(my_z * kZPlane + (my_all - my_z) * (T9 ? kZPlane : kXPlane));
         int i = 0;
         for (; i < ntile; ++i) {
             const int s = i % S, tile = first + i * stride;
@@ -945,7 +952,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) wgrad3_kernel(const WgradPar
             uint8_t *st = smem + (size_t)s * stage_bytes;
             if (lane == 0) tc::mbar_expect_tx(&full[s], tx_bytes);
             __syncwarp();   // the transaction count is raised before any copy lands
-            for (int q = lane; q < nplanes; q += 32) {
+            for (int q = warp + kWgradLoadWarps * lane; q < nplanes; q += 32 * kWgradLoadWarps) {
                 if (q < nz) {
                     // output gradient: staged row j = image row y0 - 1 + j;
                     // nine-tap form: copy kx from pixel x0 + 1 - kx
@@ -972,7 +979,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) wgrad3_kernel(const WgradPar
         if (lane == 0)
             for (int s = 0; s < S && s < i; ++s)
                 tc::mbar_wait(&full[s], (uint32_t)((i - s + S - 1) / S - 1) & 1u, kWaitIter);
-    } else if (warp == 1) {
+    } else if (warp == kWgradLoadWarps) {
         // ---- MMA issue (one thread) ----
         if (lane == 0) {
             const uint32_t idesc = tc::idesc_bf16(kPx, N) | (1u << 15) | (1u << 16);   // A and B MN-major
@@ -1014,7 +1021,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) wgrad3_kernel(const WgradPar
     } else {
         // ---- bias warps: the tile's centre gradient rows (staged rows 1..R;
         // the nine-tap form's unshifted copy kx = 1) ----
-        const int px = tid - 64;
+        const int px = tid - 32 * (kWgradLoadWarps + 1);
         for (int i = 0; i < ntile; ++i) {
             const int s = i % S;
             bool got = true;
@@ -1047,8 +1054,8 @@ __global__ void __launch_bounds__(kWgradThreads, 1) wgrad3_kernel(const WgradPar
     float *out = P.partial + (size_t)blockIdx.x * (9 * P.cin * P.cout + P.cout);
     if (!ok) {
         if (tid == 0) atomicExch(P.err, 1);
-    } else if (ntile >= 1 && warp >= 2) {
-        const int bw = warp - 2;
+    } else if (ntile >= 1 && warp > kWgradLoadWarps) {
+        const int bw = warp - kWgradLoadWarps - 1;
         // bias: lanes, then the four warps in a fixed order
 #pragma unroll
         for (int j = 0; j < 8 * ZC; ++j) {
@@ -1088,7 +1095,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) wgrad3_kernel(const WgradPar
     }
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 1) tc::tmem_dealloc(tbase, cols);
+    if (warp == kWgradLoadWarps) tc::tmem_dealloc(tbase, cols);
 }
 
 template <int ZC, bool T9>
