@@ -62,9 +62,9 @@ constexpr int kBufLvl[NBUF] = {0, 0, 0, 1, 1, 1, 2, 2, 2, 1, 1, 1, 0, 0,
 
 size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
-// Workspace: [error flag][packed weights per conv: fwd, dgrad][buffers][partials]
+// Workspace: [error flag][packed weights per conv: fwd, dgrad][buffers][partials per layer]
 struct Layout {
-    size_t pack_fwd[kLayers], pack_dg[kLayers], buf[NBUF], partial, partial2, total;
+    size_t pack_fwd[kLayers], pack_dg[kLayers], buf[NBUF], partial[kLayers], total;
     int steps_fwd[kLayers], steps_dg[kLayers];
 };
 
@@ -76,19 +76,27 @@ constexpr int kSrc1[kLayers] = {0, 0, 0, 0, 0, 0, 0, 2, 0, 0, 1, 0};
 // pyramid level of each layer's input (0 full, 1 half, 2 quarter)
 constexpr int kLvl[kLayers] = {0, 0, 1, 1, 2, 2, 2, 1, 1, 1, 0, 0};
 
-size_t partial_floats(int B, int H, int W)
+// The weight gradient of a 3x3 layer, without its pointers.
+WgradParams wgrad_params(int cin, int cout, int xc0, int xc1, int H, int W)
 {
-    size_t m = 0;
-    for (int l = 0; l < kLayers; ++l) {
-        const LayerDef &d = kDef[l];
-        const int h = H >> kLvl[l], w = W >> kLvl[l];
-        size_t n = 0;
-        if (d.kind == CONV) n = wgrad_partial_floats(B, h, w, d.cin, d.cout);
-        else if (d.kind == TCONV) n = reduce_floats(d.cin * d.cout + d.cout, (int)tconv_blocks(d.cin, h, w, B));
-        else n = reduce_floats(54, (int)head_blocks((size_t)B * H * W));
-        m = n > m ? n : m;
-    }
-    return m;
+    WgradParams P{};
+    P.xc0 = xc0;
+    P.xc1 = xc1;
+    P.zc = chunks(cout);
+    P.cin = cin;
+    P.cout = cout;
+    P.H = H;
+    P.W = W;
+    return P;
+}
+
+// Partial rows of layer l's parameter gradient.
+int partial_rows(int l, int B, int H, int W)
+{
+    const LayerDef &d = kDef[l];
+    const int h = H >> kLvl[l], w = W >> kLvl[l];
+    if (d.kind == CONV) return wgrad_partial_rows(wgrad_params(d.cin, d.cout, kSrc0[l], kSrc1[l], h, w), B);
+    return (int)(d.kind == TCONV ? tconv_blocks(d.cin, h, w, B) : head_blocks((size_t)B * H * W));
 }
 
 Layout layout(int B, int H, int W)
@@ -111,10 +119,10 @@ Layout layout(int B, int H, int W)
         L.buf[i] = o;
         o += align256((size_t)B * (H >> kBufLvl[i]) * (W >> kBufLvl[i]) * kBufCh[i] * 2);
     }
-    L.partial = o;
-    o += align256(partial_floats(B, H, W) * sizeof(float));
-    L.partial2 = o;   // the weight gradients' partials (companion stream)
-    o += align256(partial_floats(B, H, W) * sizeof(float));
+    for (int l = 0; l < kLayers; ++l) {
+        L.partial[l] = o;
+        o += align256((size_t)partial_rows(l, B, H, W) * param_size(kDef[l]) * sizeof(float));
+    }
     L.total = o;
     return L;
 }
@@ -130,8 +138,7 @@ struct Ctx {
     bool stacked_for(int nout) const { return stacked && nout == 16; }
     __nv_bfloat16 *buf(Buf b) const { return reinterpret_cast<__nv_bfloat16 *>(ws + L.buf[b]); }
     int *err() const { return reinterpret_cast<int *>(ws); }
-    float *partial() const { return reinterpret_cast<float *>(ws + L.partial); }
-    float *partial2() const { return reinterpret_cast<float *>(ws + L.partial2); }
+    float *partial(int l) const { return reinterpret_cast<float *>(ws + L.partial[l]); }
     const float *w(int l) const { return params + param_offset(l); }
     const float *b(int l) const { return params + param_offset(l) + weight_count(l); }
 };
@@ -196,26 +203,27 @@ cudaError_t conv(const Ctx &c, int l, bool dgrad, int lvl, Buf s0, int c0, Buf s
     return launch_conv3x3(P, c.B, nout_of(dgrad ? d.cin : d.cout), c.st);
 }
 
-// Weight and bias gradient of layer l on stream `st` with partial buffer `part`.
-cudaError_t wgrad(const Ctx &c, float *grads, int l, int lvl, Buf x0, int xc0, Buf x1, int xc1, Buf dz,
-                  cudaStream_t st, float *part)
+// Partial sums of the weight and bias gradient of layer l, on stream `st`.
+cudaError_t wgrad(const Ctx &c, int l, Buf x0, Buf x1, Buf dz, cudaStream_t st)
 {
     const LayerDef &d = kDef[l];
-    WgradParams P{};
+    WgradParams P = wgrad_params(d.cin, d.cout, kSrc0[l], kSrc1[l], c.H >> kLvl[l], c.W >> kLvl[l]);
     P.x0 = c.buf(x0);
-    P.x1 = xc1 ? c.buf(x1) : nullptr;
-    P.xc0 = xc0;
-    P.xc1 = xc1;
+    P.x1 = P.xc1 ? c.buf(x1) : nullptr;
     P.dz = c.buf(dz);
-    P.zc = chunks(d.cout);
-    P.cin = d.cin;
-    P.cout = d.cout;
-    P.partial = part;
-    P.H = c.H >> lvl;
-    P.W = c.W >> lvl;
+    P.partial = c.partial(l);
     P.err = c.err();
-    CD_TRY(launch_wgrad(P, c.B, st));
-    return launch_reduce(part, grads + param_offset(l), param_size(d), wgrad_partial_rows(P, c.B), st);
+    return launch_wgrad(P, c.B, st);
+}
+
+// Every parameter gradient from its layer's partial sums.
+cudaError_t reduce_all(const Ctx &c, float *grads)
+{
+    ReduceJobs J{};
+    for (int l = 0; l < kLayers; ++l)
+        J.job[J.n++] = ReduceJob{c.partial(l), grads + param_offset(l), param_size(kDef[l]),
+                                 partial_rows(l, c.B, c.H, c.W)};
+    return launch_reduce(J, c.st);
 }
 
 // A companion stream per caller stream (and device) for the weight
@@ -288,64 +296,58 @@ cudaError_t backward(const float *gband, const float *galpha, const float *param
     const size_t n0 = (size_t)B * H * W;
     Side *side = side_stream(st);
     // weight gradient of layer l, forked onto the companion stream when there is one
-    auto wg = [&](int l, int lvl, Buf x0, int xc0, Buf x1, int xc1, Buf dz) -> cudaError_t {
-        if (!side) return wgrad(c, grads, l, lvl, x0, xc0, x1, xc1, dz, st, c.partial2());
+    auto wg = [&](int l, Buf x0, Buf x1, Buf dz) -> cudaError_t {
+        if (!side) return wgrad(c, l, x0, x1, dz, st);
         CD_TRY(cudaEventRecord(side->fork, st));
         CD_TRY(cudaStreamWaitEvent(side->s, side->fork, 0));
-        return wgrad(c, grads, l, lvl, x0, xc0, x1, xc1, dz, side->s, c.partial2());
+        return wgrad(c, l, x0, x1, dz, side->s);
     };
     auto body = [&]() -> cudaError_t {
         CD_TRY(pack_all(c, true));
         // head
-        CD_TRY(launch_head_bwd(c.buf(C51), c.w(11), c.b(11), gband, galpha, c.buf(DZ10), c.partial(), n0, st));
-        CD_TRY(launch_reduce(c.partial(), grads + param_offset(11), 54, (int)head_blocks(n0), st));
+        CD_TRY(launch_head_bwd(c.buf(C51), c.w(11), c.b(11), gband, galpha, c.buf(DZ10), c.partial(11), n0, st));
         // L10: 24 -> 8 at full resolution; input gradient splits into c4_3 and the c1_2 skip
-        CD_TRY(wg(10, 0, C43, 2, C12, 1, DZ10));
+        CD_TRY(wg(10, C43, C12, DZ10));
         CD_TRY(conv(c, 10, true, 0, DZ10, 1, NONE, 0, DC43, 2, DSK1, 1, NONE, NONE, NONE));
         // L9: transposed conv half -> full
-        CD_TRY(launch_tconv_bwd(16, 16, c.buf(C42), c.buf(DC43), c.w(9), c.buf(DZ8), c.partial(), H >> 1, W >> 1, B,
+        CD_TRY(launch_tconv_bwd(16, 16, c.buf(C42), c.buf(DC43), c.w(9), c.buf(DZ8), c.partial(9), H >> 1, W >> 1, B,
                                 st));
-        CD_TRY(launch_reduce(c.partial(), grads + param_offset(9), param_size(kDef[9]),
-                             (int)tconv_blocks(16, H >> 1, W >> 1, B), st));
         // L8
-        CD_TRY(wg(8, 1, C41, 2, NONE, 0, DZ8));
+        CD_TRY(wg(8, C41, NONE, DZ8));
         CD_TRY(conv(c, 8, true, 1, DZ8, 2, NONE, 0, DZ7, 2, NONE, 0, C41, NONE, NONE));
         // L7: 48 -> 16; input gradient splits into c3_3 and the c2_2 skip
-        CD_TRY(wg(7, 1, C33, 4, C22, 2, DZ7));
+        CD_TRY(wg(7, C33, C22, DZ7));
         CD_TRY(conv(c, 7, true, 1, DZ7, 2, NONE, 0, DC33, 4, DSK2, 2, NONE, NONE, NONE));
         // L6: transposed conv quarter -> half
-        CD_TRY(launch_tconv_bwd(32, 32, c.buf(C32), c.buf(DC33), c.w(6), c.buf(DZ5), c.partial(), H >> 2, W >> 2, B,
+        CD_TRY(launch_tconv_bwd(32, 32, c.buf(C32), c.buf(DC33), c.w(6), c.buf(DZ5), c.partial(6), H >> 2, W >> 2, B,
                                 st));
-        CD_TRY(launch_reduce(c.partial(), grads + param_offset(6), param_size(kDef[6]),
-                             (int)tconv_blocks(32, H >> 2, W >> 2, B), st));
         // L5, L4
-        CD_TRY(wg(5, 2, C31, 4, NONE, 0, DZ5));
+        CD_TRY(wg(5, C31, NONE, DZ5));
         CD_TRY(conv(c, 5, true, 2, DZ5, 4, NONE, 0, DZ4, 4, NONE, 0, C31, NONE, NONE));
-        CD_TRY(wg(4, 2, C23, 2, NONE, 0, DZ4));
+        CD_TRY(wg(4, C23, NONE, DZ4));
         CD_TRY(conv(c, 4, true, 2, DZ4, 4, NONE, 0, DC23, 2, NONE, 0, NONE, NONE, NONE));
         // pool of c2_2 + skip, ReLU of c2_2
         CD_TRY(launch_pool_bwd(16, c.buf(C22), c.buf(C23), c.buf(DC23), c.buf(DSK2), c.buf(DZ3), H >> 1, W >> 1, B,
                                st));
         // L3, L2
-        CD_TRY(wg(3, 1, C21, 2, NONE, 0, DZ3));
+        CD_TRY(wg(3, C21, NONE, DZ3));
         CD_TRY(conv(c, 3, true, 1, DZ3, 2, NONE, 0, DZ2, 2, NONE, 0, C21, NONE, NONE));
-        CD_TRY(wg(2, 1, C13, 1, NONE, 0, DZ2));
+        CD_TRY(wg(2, C13, NONE, DZ2));
         CD_TRY(conv(c, 2, true, 1, DZ2, 2, NONE, 0, DC13, 1, NONE, 0, NONE, NONE, NONE));
         // pool of c1_2 + skip, ReLU of c1_2
         CD_TRY(launch_pool_bwd(8, c.buf(C12), c.buf(C13), c.buf(DC13), c.buf(DSK1), c.buf(DZ1), H, W, B, st));
         // L1, L0
-        CD_TRY(wg(1, 0, C11, 1, NONE, 0, DZ1));
+        CD_TRY(wg(1, C11, NONE, DZ1));
         CD_TRY(conv(c, 1, true, 0, DZ1, 1, NONE, 0, DZ0, 1, NONE, 0, C11, NONE, NONE));
-        return wg(0, 0, X0, 2, NONE, 0, DZ0);
+        return wg(0, X0, NONE, DZ0);
     };
-    const cudaError_t e = body();
+    cudaError_t e = body();
     if (side) {   // join, also after a failed launch, so no fork is left open
         const cudaError_t e1 = cudaEventRecord(side->join, side->s);
         const cudaError_t e2 = cudaStreamWaitEvent(st, side->join, 0);
-        if (e == cudaSuccess && e1 != cudaSuccess) return e1;
-        if (e == cudaSuccess && e2 != cudaSuccess) return e2;
+        if (e == cudaSuccess) e = e1 != cudaSuccess ? e1 : e2;
     }
-    return e;
+    return e == cudaSuccess ? reduce_all(c, grads) : e;
 }
 
 size_t conv_layer_workspace(int cin, int cout)
@@ -393,26 +395,24 @@ cudaError_t conv_layer(const float *w, const float *bias, const __nv_bfloat16 *x
 
 size_t wgrad_layer_workspace(int cin, int cout, int B, int H, int W)
 {
-    return 256 + align256(wgrad_partial_floats(B, H, W, cin, cout) * sizeof(float));
+    const int rows = wgrad_partial_rows(wgrad_params(cin, cout, chunks(cin), 0, H, W), B);
+    return 256 + align256((size_t)rows * (9 * cin * cout + cout) * sizeof(float));
 }
 
 cudaError_t wgrad_layer(const __nv_bfloat16 *x, const __nv_bfloat16 *dz, float *grad, int cin, int cout, int B,
                         int H, int W, void *ws, cudaStream_t st)
 {
     uint8_t *base = static_cast<uint8_t *>(ws);
-    WgradParams P{};
+    WgradParams P = wgrad_params(cin, cout, chunks(cin), 0, H, W);
     P.x0 = x;
-    P.xc0 = chunks(cin);
     P.dz = dz;
-    P.zc = chunks(cout);
-    P.cin = cin;
-    P.cout = cout;
     P.partial = reinterpret_cast<float *>(base + 256);
-    P.H = H;
-    P.W = W;
     P.err = reinterpret_cast<int *>(base);
     CD_TRY(launch_wgrad(P, B, st));
-    return launch_reduce(P.partial, grad, 9 * cin * cout + cout, wgrad_partial_rows(P, B), st);
+    ReduceJobs J{};
+    J.n = 1;
+    J.job[0] = ReduceJob{P.partial, grad, 9 * cin * cout + cout, wgrad_partial_rows(P, B)};
+    return launch_reduce(J, st);
 }
 
 cudaError_t adam(float *w, const float *g, float *m, float *v, int n, int *step, float lr, float b1, float b2,

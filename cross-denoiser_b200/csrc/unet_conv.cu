@@ -1233,12 +1233,10 @@ cudaError_t launch_pack(const float *w, __nv_bfloat16 *dst, const PackTable &T, 
 size_t wgrad_tiles(int B, int H, int W) { return (size_t)B * ((W + kPx - 1) / kPx) * ((H + kWgradRows - 1) / kWgradRows); }
 
 
-static int sm_count()
-{
-    int dev = 0, n = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n;
-}
+// CTAs of a layer's weight gradient: one per SM of a 148-SM part (a constant,
+// so that neither the workspace's size nor the sums' order depend on the
+// device).
+constexpr int kWgradCtas = 148;
 
 // The persistent kernel takes every layer whose (ky, cout) fit N
 // (zc <= 4) and whose input channels fit M (at most 16 chunks).  The
@@ -1263,13 +1261,7 @@ int wgrad_partial_rows(const WgradParams &P, int B)
     if (!wgrad3_fits(P)) return (int)wgrad_tiles(B, P.H, P.W);
     const Wgrad3Plan p = wgrad3_plan_of(P);
     const int tiles = B * ((P.W + kPx - 1) / kPx) * ((P.H + p.R - 1) / p.R);
-    return tiles < sm_count() ? tiles : sm_count();
-}
-
-size_t wgrad_partial_floats(int B, int H, int W, int cin, int cout)
-{
-    const size_t t = wgrad_tiles(B, H, W);
-    return reduce_floats(9 * cin * cout + cout, (int)(t > 1024 ? t : 1024));
+    return tiles < kWgradCtas ? tiles : kWgradCtas;
 }
 
 cudaError_t launch_wgrad(const WgradParams &P, int B, cudaStream_t st)

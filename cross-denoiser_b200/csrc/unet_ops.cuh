@@ -23,10 +23,18 @@ cudaError_t launch_head_bwd(const __nv_bfloat16 *x, const float *K, const float 
 cudaError_t launch_pool_bwd(int C, const __nv_bfloat16 *act, const __nv_bfloat16 *pooled,
                             const __nv_bfloat16 *dpool, const __nv_bfloat16 *dskip, __nv_bfloat16 *dz, int H, int W,
                             int B, cudaStream_t st);
-// Sum per-tile partials partial[t * n + j] over t into out[j] (fixed order).
-// The partial buffer holds reduce_floats(n, tiles) floats.
-size_t reduce_floats(int n, int tiles);
-cudaError_t launch_reduce(float *partial, float *out, int n, int tiles, cudaStream_t st);
+// Sums of partial rows: out[j] = sum over t of partial[t * n + j] (fixed order), per job.
+constexpr int kMaxReduceJobs = 12;
+struct ReduceJob {
+    const float *partial;
+    float *out;
+    int n, rows;
+};
+struct ReduceJobs {
+    ReduceJob job[kMaxReduceJobs];
+    int n;
+};
+cudaError_t launch_reduce(const ReduceJobs &J, cudaStream_t st);
 cudaError_t launch_adam(float *w, const float *g, float *m, float *v, int n, int *step, float lr, float b1, float b2,
                         float eps, cudaStream_t st);
 
