@@ -30,6 +30,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include "cd_common.cuh"
+#include "launch.cuh"
 #include "tc_sm100.cuh"
 #include "unet.cuh"
 #include "unet_ops.cuh"
@@ -214,12 +215,14 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const ConvParams P)
 
     // per input source, planes [row][chunk][131 px][8 ch] (zeros outside the
     // image), and the packed weights: bulk copies on one mbarrier
-    if (warp == 0) tc::tmem_alloc(tslot, kCols);
     if (tid == 0) {
         tc::mbar_init(bar, 1);
         tc::fence_async_smem();
     }
+    chain_wait();
+    if (warp == 0) tc::tmem_alloc(tslot, kCols);
     __syncthreads();   // barrier initialised before the copies are issued and waited on
+    chain_next();
     if (warp == 0) {
         const int lane = tid & 31, nch = P.c0 + P.c1;
         if (lane == 0) {
@@ -334,8 +337,7 @@ cudaError_t launch_t(const ConvParams &P, int B, cudaStream_t st)
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     dim3 grid((P.W + kPx - 1) / kPx, (P.H + R - 1) / R, B);
-    conv3x3_kernel<NOUT, R, KYN, NST><<<grid, 128, smem, st>>>(P);
-    return cudaGetLastError();
+    return launch_chained(conv3x3_kernel<NOUT, R, KYN, NST>, grid, 128, smem, st, P);
 }
 
 // Per-row form with the step count as a template parameter for the
@@ -420,6 +422,7 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
     uint64_t *wbar = tempty + 2;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(wbar + 1);
 
+    chain_wait();
     if (warp == 1) tc::tmem_alloc(tslot, kCols);
     if (tid == 0) {
         for (int s = 0; s < S; ++s) {
@@ -437,6 +440,7 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
     __syncthreads();
     tc::fence_after_sync();
     const uint32_t tbase = *tslot;
+    chain_next();
     // both accumulator buffers start at zero (every MMA accumulates)
     if (warp >= 2) {
         const uint32_t lanes = tbase + ((uint32_t)((warp & 3) * 32) << 16);
@@ -594,8 +598,8 @@ cudaError_t launch_pipe_t(const ConvParams &P, const ConvPipePlan &pl, int per_s
     int dev = 0, nsm = 148;
     if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     const int grid = ntiles < per_sm * nsm ? ntiles : per_sm * nsm;
-    conv3x3_pipe_kernel<NOUT, R, NST><<<grid, kPipeThreads, pl.smem, st>>>(P, pl, ntx, nty, ntiles);
-    return cudaGetLastError();
+    return launch_chained(conv3x3_pipe_kernel<NOUT, R, NST>, grid, kPipeThreads, pl.smem, st, P, pl, ntx, nty,
+                          ntiles);
 }
 
 // The step counts of the network's 16-output layers: 2 (one chunk), 3 (a
@@ -646,12 +650,16 @@ __device__ __forceinline__ void pack_one(const float *__restrict__ w, __nv_bfloa
 
 __global__ void pack_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ dst, const PackTable T)
 {
+    chain_wait();
+    chain_next();
     pack_one(w, dst, T, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // grid row j packs job j
 __global__ void pack_jobs_kernel(const __grid_constant__ PackJobs J)
 {
+    chain_wait();
+    chain_next();
     const PackJob &j = J.job[blockIdx.y];
     pack_one(j.w, j.dst, j.T, blockIdx.x * blockDim.x + threadIdx.x);
 }
@@ -1219,15 +1227,13 @@ cudaError_t launch_pack_jobs(const PackJobs &J, cudaStream_t st)
         const int n = J.job[j].T.nsteps * 2 * J.job[j].T.nout * (J.job[j].T.stacked ? 3 : 1) * 8;
         most = n > most ? n : most;
     }
-    pack_jobs_kernel<<<dim3((most + 255) / 256, J.n), 256, 0, st>>>(J);
-    return cudaGetLastError();
+    return launch_chained(pack_jobs_kernel, dim3((most + 255) / 256, J.n), 256, 0, st, J);
 }
 
 cudaError_t launch_pack(const float *w, __nv_bfloat16 *dst, const PackTable &T, cudaStream_t st)
 {
     const int n = T.nsteps * 2 * T.nout * (T.stacked ? 3 : 1) * 8;
-    pack_kernel<<<(n + 255) / 256, 256, 0, st>>>(w, dst, T);
-    return cudaGetLastError();
+    return launch_chained(pack_kernel, (n + 255) / 256, 256, 0, st, w, dst, T);
 }
 
 size_t wgrad_tiles(int B, int H, int W) { return (size_t)B * ((W + kPx - 1) / kPx) * ((H + kWgradRows - 1) / kWgradRows); }

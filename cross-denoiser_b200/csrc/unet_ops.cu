@@ -17,6 +17,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include "cd_common.cuh"
+#include "launch.cuh"
 #include "unet.cuh"
 #include "unet_ops.cuh"
 
@@ -51,6 +52,8 @@ __global__ void __launch_bounds__(256) pack_input_kernel(const float *__restrict
                                                          const float *__restrict__ e, __nv_bfloat16 *__restrict__ x,
                                                          size_t n, int W)
 {
+    chain_wait();
+    chain_next();
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     const int row = (int)(p / W), px = (int)(p - (size_t)row * W);
@@ -76,6 +79,8 @@ __global__ void __launch_bounds__(256) tconv_fwd_kernel(const __nv_bfloat16 *__r
                                                         const float *__restrict__ K, const float *__restrict__ bias,
                                                         __nv_bfloat16 *__restrict__ out, int Hi, int Wi, int B)
 {
+    chain_wait();
+    chain_next();
     __shared__ __align__(16) float sK[CO * CI + CO];
     for (int i = threadIdx.x; i < CO * CI + CO; i += blockDim.x) sK[i] = i < CO * CI ? K[i] : bias[i - CO * CI];
     __syncthreads();
@@ -123,6 +128,8 @@ __global__ void __launch_bounds__(kN) tconv_bwd_kernel(const __nv_bfloat16 *__re
                                                         __nv_bfloat16 *__restrict__ dz_in, float *__restrict__ partial,
                                                         int Hi, int Wi, int B)
 {
+    chain_wait();
+    chain_next();
     // dK in 4 x 4 register tiles: kTiles tiles cover CO x CI, and the
     // threads split into kGroups pixel groups, each summing its share of a
     // chunk's pixels (in order) into every tile; the groups' sums are added
@@ -249,6 +256,8 @@ __global__ void __launch_bounds__(256) head_fwd_kernel(const __nv_bfloat16 *__re
                                                        const float *__restrict__ bias, float *__restrict__ band,
                                                        float *__restrict__ alpha, size_t n)
 {
+    chain_wait();
+    chain_next();
     __shared__ float sK[54];
     __shared__ __align__(16) float sb[256 * 5];   // the block's band values, written out as float4
     const int tid = threadIdx.x;
@@ -297,6 +306,8 @@ __global__ void __launch_bounds__(kHeadThreads) head_bwd_kernel(const __nv_bfloa
                                                                 __nv_bfloat16 *__restrict__ dz,
                                                                 float *__restrict__ partial, size_t n)
 {
+    chain_wait();
+    chain_next();
     __shared__ float sK[54];
     __shared__ float red[kHeadThreads / 32][54];
     const int tid = threadIdx.x;
@@ -367,6 +378,8 @@ __global__ void __launch_bounds__(256) pool_bwd_kernel(const __nv_bfloat16 *__re
                                                        const __nv_bfloat16 *__restrict__ dskip,
                                                        __nv_bfloat16 *__restrict__ dz, int H, int W, int B)
 {
+    chain_wait();
+    chain_next();
     constexpr int NC = C / 8;
     const int PH = H / 2, PW = W / 2;
     const size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -414,6 +427,8 @@ constexpr int kReduceWarps = 32;
 
 __global__ void __launch_bounds__(32 * kReduceWarps) reduce_kernel(const __grid_constant__ ReduceJobs J)
 {
+    chain_wait();
+    chain_next();
     __shared__ float red[kReduceWarps][33];
     int k = 0, blk = blockIdx.x;
     while (k + 1 < J.n && blk >= (J.job[k].n + 31) / 32) blk -= (J.job[k++].n + 31) / 32;
@@ -443,6 +458,8 @@ __global__ void __launch_bounds__(256) adam_kernel(float *__restrict__ w, const 
                                                    const int *__restrict__ step, float lr, float b1, float b2,
                                                    float eps)
 {
+    chain_wait();
+    chain_next();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float t = (float)(*step + 1);
@@ -455,15 +472,18 @@ __global__ void __launch_bounds__(256) adam_kernel(float *__restrict__ w, const 
     w[i] -= (mi * lr_t) / (sqrtf(vi) + eps);
 }
 
-__global__ void step_kernel(int *step) { *step += 1; }
+__global__ void step_kernel(int *step)
+{
+    chain_wait();
+    *step += 1;
+}
 
 }  // namespace
 
 cudaError_t launch_pack_input(const float *a, const float *b, const float *c, const float *d, const float *e,
                               __nv_bfloat16 *x, size_t n, int W, cudaStream_t st)
 {
-    pack_input_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a, b, c, d, e, x, n, W);
-    return cudaGetLastError();
+    return launch_chained(pack_input_kernel, (unsigned)((n + 255) / 256), 256, 0, st, a, b, c, d, e, x, n, W);
 }
 
 cudaError_t launch_tconv_fwd(int ci, int co, const __nv_bfloat16 *in, const float *K, const float *bias,
@@ -471,10 +491,11 @@ cudaError_t launch_tconv_fwd(int ci, int co, const __nv_bfloat16 *in, const floa
 {
     const size_t n = (size_t)B * Hi * Wi;
     const unsigned g = (unsigned)((n + 255) / 256);
-    if (ci == 32 && co == 32) tconv_fwd_kernel<32, 32><<<g, 256, 0, st>>>(in, K, bias, out, Hi, Wi, B);
-    else if (ci == 16 && co == 16) tconv_fwd_kernel<16, 16><<<g, 256, 0, st>>>(in, K, bias, out, Hi, Wi, B);
-    else return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    if (ci == 32 && co == 32) return launch_chained(tconv_fwd_kernel<32, 32>, g, 256, 0, st, in, K, bias, out, Hi,
+                                                    Wi, B);
+    if (ci == 16 && co == 16) return launch_chained(tconv_fwd_kernel<16, 16>, g, 256, 0, st, in, K, bias, out, Hi,
+                                                    Wi, B);
+    return cudaErrorInvalidValue;
 }
 
 // pixels per block of the transposed-conv backward (static shared memory < 48 KB)
@@ -494,18 +515,17 @@ cudaError_t launch_tconv_bwd(int ci, int co, const __nv_bfloat16 *in, const __nv
                              __nv_bfloat16 *dz_in, float *partial, int Hi, int Wi, int B, cudaStream_t st)
 {
     const unsigned g = (unsigned)tconv_blocks(ci, Hi, Wi, B);
-    if (ci == 32 && co == 32) tconv_bwd_kernel<32, 32, 64><<<g, 64, 0, st>>>(in, dout, K, dz_in, partial, Hi, Wi, B);
-    else if (ci == 16 && co == 16)
-        tconv_bwd_kernel<16, 16, 128><<<g, 128, 0, st>>>(in, dout, K, dz_in, partial, Hi, Wi, B);
-    else return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    if (ci == 32 && co == 32) return launch_chained(tconv_bwd_kernel<32, 32, 64>, g, 64, 0, st, in, dout, K, dz_in,
+                                                    partial, Hi, Wi, B);
+    if (ci == 16 && co == 16)
+        return launch_chained(tconv_bwd_kernel<16, 16, 128>, g, 128, 0, st, in, dout, K, dz_in, partial, Hi, Wi, B);
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_head_fwd(const __nv_bfloat16 *x, const float *K, const float *bias, float *band, float *alpha,
                             size_t n, cudaStream_t st)
 {
-    head_fwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(x, K, bias, band, alpha, n);
-    return cudaGetLastError();
+    return launch_chained(head_fwd_kernel, (unsigned)((n + 255) / 256), 256, 0, st, x, K, bias, band, alpha, n);
 }
 
 size_t head_blocks(size_t n)
@@ -517,8 +537,8 @@ size_t head_blocks(size_t n)
 cudaError_t launch_head_bwd(const __nv_bfloat16 *x, const float *K, const float *bias, const float *gband,
                             const float *galpha, __nv_bfloat16 *dz, float *partial, size_t n, cudaStream_t st)
 {
-    head_bwd_kernel<<<(unsigned)head_blocks(n), kHeadThreads, 0, st>>>(x, K, bias, gband, galpha, dz, partial, n);
-    return cudaGetLastError();
+    return launch_chained(head_bwd_kernel, (unsigned)head_blocks(n), kHeadThreads, 0, st, x, K, bias, gband, galpha,
+                          dz, partial, n);
 }
 
 cudaError_t launch_pool_bwd(int C, const __nv_bfloat16 *act, const __nv_bfloat16 *pooled,
@@ -528,10 +548,9 @@ cudaError_t launch_pool_bwd(int C, const __nv_bfloat16 *act, const __nv_bfloat16
     if ((H | W) & 1) return cudaErrorInvalidValue;   // the network's levels are even-sized
     const size_t n = (size_t)B * (H / 2) * (W / 2);
     const unsigned g = (unsigned)((n + 255) / 256);
-    if (C == 8) pool_bwd_kernel<8><<<g, 256, 0, st>>>(act, pooled, dpool, dskip, dz, H, W, B);
-    else if (C == 16) pool_bwd_kernel<16><<<g, 256, 0, st>>>(act, pooled, dpool, dskip, dz, H, W, B);
-    else return cudaErrorInvalidValue;
-    return cudaGetLastError();
+    if (C == 8) return launch_chained(pool_bwd_kernel<8>, g, 256, 0, st, act, pooled, dpool, dskip, dz, H, W, B);
+    if (C == 16) return launch_chained(pool_bwd_kernel<16>, g, 256, 0, st, act, pooled, dpool, dskip, dz, H, W, B);
+    return cudaErrorInvalidValue;
 }
 
 cudaError_t launch_reduce(const ReduceJobs &J, cudaStream_t st)
@@ -539,16 +558,14 @@ cudaError_t launch_reduce(const ReduceJobs &J, cudaStream_t st)
     if (J.n < 1 || J.n > kMaxReduceJobs) return cudaErrorInvalidValue;
     int blocks = 0;
     for (int k = 0; k < J.n; ++k) blocks += (J.job[k].n + 31) / 32;
-    reduce_kernel<<<blocks, 32 * kReduceWarps, 0, st>>>(J);
-    return cudaGetLastError();
+    return launch_chained(reduce_kernel, blocks, 32 * kReduceWarps, 0, st, J);
 }
 
 cudaError_t launch_adam(float *w, const float *g, float *m, float *v, int n, int *step, float lr, float b1, float b2,
                         float eps, cudaStream_t st)
 {
-    adam_kernel<<<(n + 255) / 256, 256, 0, st>>>(w, g, m, v, n, step, lr, b1, b2, eps);
-    step_kernel<<<1, 1, 0, st>>>(step);
-    return cudaGetLastError();
+    const cudaError_t e = launch_chained(adam_kernel, (n + 255) / 256, 256, 0, st, w, g, m, v, n, step, lr, b1, b2, eps);
+    return e != cudaSuccess ? e : launch_chained(step_kernel, 1, 1, 0, st, step);
 }
 
 }  // namespace unet
