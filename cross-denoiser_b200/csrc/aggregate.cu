@@ -16,6 +16,7 @@
 // pass gives the filtered frame, the loss and dL/dband.
 #include <cuda_runtime.h>
 #include "cd_common.cuh"
+#include "launch.cuh"
 #include "filter_sweep.cuh"
 
 namespace cd {
@@ -109,6 +110,8 @@ CD_DEV void block_partial(float v, float *partial, int nthreads)
 __global__ void __launch_bounds__(1024) loss_reduce_kernel(const float *__restrict__ partial, int n,
                                                            float inv_n, float *__restrict__ avg)
 {
+    chain_wait();
+    chain_next();
     __shared__ float red[32];
     float v = 0.f;
     for (int i = threadIdx.x; i < n; i += blockDim.x) v += partial[i];
@@ -125,6 +128,8 @@ __global__ void __launch_bounds__(1024) loss_reduce_kernel(const float *__restri
 __global__ void __launch_bounds__(256) log1p_kernel(const float *__restrict__ a, const float *__restrict__ b,
                                                     float *__restrict__ ya, float *__restrict__ yb, size_t n)
 {
+    chain_wait();
+    chain_next();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
         ya[i] = log1pf(__ldg(a + i));
@@ -139,6 +144,8 @@ constexpr int kLogVec = 2;
 __global__ void __launch_bounds__(256) log1p4_kernel(const float4 *__restrict__ a, const float4 *__restrict__ b,
                                                      float4 *__restrict__ ya, float4 *__restrict__ yb, size_t n4)
 {
+    chain_wait();
+    chain_next();
     const size_t i0 = ((size_t)blockIdx.x * kLogVec) * blockDim.x + threadIdx.x;
     float4 va[kLogVec], vb[kLogVec];
 #pragma unroll
@@ -169,6 +176,8 @@ struct AggPtrs {
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) aggregation_kernel(AggPtrs P, int H, int W, float inv_n)
 {
+    chain_wait();
+    chain_next();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
     const bool ok = x < W && y < H;
     float loss = 0.f;
@@ -265,6 +274,8 @@ __global__ void __launch_bounds__(256, 2) filter_aggregate_kernel(
     const float *__restrict__ normal, const float *__restrict__ band, AggPtrs P,
     float *__restrict__ gband, int H, int W, int hw_rt, float inv_n)
 {
+    chain_wait();
+    chain_next();
     extern __shared__ ulonglong2 tile[];
     const int hw = HW > 0 ? HW : hw_rt;
     const int tw = fsw::kBX + 2 * hw, th = fsw::kBY + 2 * hw;
@@ -298,13 +309,11 @@ cudaError_t launch_log1p(const float *a, const float *b, float *ya, float *yb, s
                                      reinterpret_cast<uintptr_t>(ya) | reinterpret_cast<uintptr_t>(yb)) & 15) == 0;
     if (vec) {
         const size_t n4 = n / 4, per = (size_t)256 * kLogVec;
-        log1p4_kernel<<<(unsigned)((n4 + per - 1) / per), 256, 0, st>>>(
-            reinterpret_cast<const float4 *>(a), reinterpret_cast<const float4 *>(b), reinterpret_cast<float4 *>(ya),
-            reinterpret_cast<float4 *>(yb), n4);
-    } else {
-        log1p_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a, b, ya, yb, n);
+        return launch_chained(log1p4_kernel, (unsigned)((n4 + per - 1) / per), 256, 0, st, reinterpret_cast<const
+                             float4 *>(a), reinterpret_cast<const float4 *>(b), reinterpret_cast<float4 *>(ya),
+                             reinterpret_cast<float4 *>(yb), n4);
     }
-    return cudaGetLastError();
+    return launch_chained(log1p_kernel, (unsigned)((n + 255) / 256), 256, 0, st, a, b, ya, yb, n);
 }
 
 cudaError_t launch_aggregation(const AggArgs &A, float *partial, float *avg, int B, int H, int W,
@@ -314,11 +323,9 @@ cudaError_t launch_aggregation(const AggArgs &A, float *partial, float *avg, int
               A.out_log, A.out, A.loss, A.g_s1, A.g_w1, A.g_s2, A.g_w2, A.g_alpha, partial};
     const float inv_n = 1.f / (3.f * (float)B * (float)H * (float)W);
     dim3 block(32, 8), grid((W + 31) / 32, (H + 7) / 8, B);
-    aggregation_kernel<<<grid, block, 0, st>>>(P, H, W, inv_n);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_chained(aggregation_kernel, grid, block, 0, st, P, H, W, inv_n);
     if (e != cudaSuccess) return e;
-    loss_reduce_kernel<<<1, 1024, 0, st>>>(partial, (int)(grid.x * grid.y * grid.z), inv_n, avg);
-    return cudaGetLastError();
+    return launch_chained(loss_reduce_kernel, 1, 1024, 0, st, partial, (int)(grid.x * grid.y * grid.z), inv_n, avg);
 }
 
 size_t filter_aggregate_smem(int win) { return fsw::smem_bytes(win / 2); }
@@ -337,8 +344,8 @@ cudaError_t launch_filter_aggregate(const float *imga, const float *imgb, const 
     auto go = [&](auto kern) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        kern<<<grid, block, smem, st>>>(imga, imgb, albedo, normal, band, P, gband, H, W, hw, inv_n);
-        return cudaGetLastError();
+        return launch_chained(kern, grid, block, smem, st, imga, imgb, albedo, normal, band, P, gband, H, W, hw,
+                              inv_n);
     };
     cudaError_t e;
     switch (hw) {
@@ -348,8 +355,7 @@ cudaError_t launch_filter_aggregate(const float *imga, const float *imgb, const 
     default: e = go(filter_aggregate_kernel<0>); break;
     }
     if (e != cudaSuccess) return e;
-    loss_reduce_kernel<<<1, 1024, 0, st>>>(partial, (int)(grid.x * grid.y * grid.z), inv_n, avg);
-    return cudaGetLastError();
+    return launch_chained(loss_reduce_kernel, 1, 1024, 0, st, partial, (int)(grid.x * grid.y * grid.z), inv_n, avg);
 }
 
 }  // namespace cd

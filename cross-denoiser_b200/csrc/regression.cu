@@ -13,6 +13,7 @@
 #include <type_traits>
 #include <cuda_runtime.h>
 #include "cd_common.cuh"
+#include "launch.cuh"
 #include "f32x2.cuh"
 #include "window_rows.cuh"
 
@@ -46,6 +47,8 @@ __global__ void __launch_bounds__(kVX * kVY) variance_kernel(const float *__rest
                                                              float *__restrict__ sda,
                                                              float *__restrict__ sdb, int H, int W)
 {
+    chain_wait();
+    chain_next();
     __shared__ __align__(16) float tile[2][kVTH][kVRow];
     const int x0 = blockIdx.x * kVX, y0 = blockIdx.y * kVY, xa = x0 - 4;
     const size_t base = (size_t)blockIdx.z * H * W;
@@ -114,6 +117,8 @@ __global__ void __launch_bounds__(256) variance_px_kernel(const float *__restric
                                                        float *__restrict__ sda,
                                                        float *__restrict__ sdb, int H, int W)
 {
+    chain_wait();
+    chain_next();
     const int cx = blockIdx.x * blockDim.x + threadIdx.x;
     const int cy = blockIdx.y * blockDim.y + threadIdx.y;
     if (cx >= W || cy >= H) return;
@@ -479,6 +484,8 @@ __host__ __device__ inline size_t regression_smem(const RowGeom &g)
 // Launch bound 8 CTAs per SM (128 registers): 706 us per 1080p
 // cross-regression, window 17, against 733 under a bound of 7, 776 under 6
 // (154 registers, 12 warps per SM) and 757 under 9 (112, spills in the sums).
+// Not launched chained (launch.cuh): the waits before its loads cost it
+// registers (256x256 cross-regression 77 against 64 us).
 template <int SP>
 __global__ void __launch_bounds__(kThreads, 8) regression_kernel(
     const float *__restrict__ imga, const float *__restrict__ imgb,
@@ -644,6 +651,8 @@ __global__ void __launch_bounds__(kRX * kRThreadRows, NP == 2 ? 4 : 1) recon_ker
     const float *__restrict__ beta, float *__restrict__ outa, float *__restrict__ outb,
     float *__restrict__ state, int H, int W, int hw, int sp, int rs)
 {
+    chain_wait();
+    chain_next();
     using namespace x2;
     extern __shared__ float4 rec[];
     constexpr int kRows = NP * kRThreadRows, kBlock = kRX * kRThreadRows;
@@ -818,12 +827,10 @@ cudaError_t launch_variance(const float *imga, const float *imgb, float *vara, f
     const bool vec = W % 4 == 0 && ((reinterpret_cast<uintptr_t>(imga) | reinterpret_cast<uintptr_t>(imgb)) & 15) == 0;
     if (vec) {
         dim3 grid((W + kVX - 1) / kVX, (H + kVY - 1) / kVY, B);
-        variance_kernel<<<grid, block, 0, st>>>(imga, imgb, vara, varb, sda, sdb, H, W);
-    } else {
-        dim3 grid((W + kVX - 1) / kVX, (H + kVY - 1) / kVY, 2 * B);
-        variance_px_kernel<<<grid, block, 0, st>>>(imga, imgb, vara, varb, sda, sdb, H, W);
+        return launch_chained(variance_kernel, grid, block, 0, st, imga, imgb, vara, varb, sda, sdb, H, W);
     }
-    return cudaGetLastError();
+    dim3 grid((W + kVX - 1) / kVX, (H + kVY - 1) / kVY, 2 * B);
+    return launch_chained(variance_px_kernel, grid, block, 0, st, imga, imgb, vara, varb, sda, sdb, H, W);
 }
 
 size_t regression_smem_bytes(int win, int sp) { return regression_smem(row_geom(win / 2, sp)); }
@@ -842,8 +849,7 @@ cudaError_t launch_regression(const float *imga, const float *imgb, const float 
         const size_t smem = regression_smem(g);
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        kern<<<grid, kThreads, smem, st>>>(imga, imgb, albedo, normal, vara, varb, sda, sdb, beta, chol, cond_limit,
-                                           fallbacks, H, W, hw, sp);
+        kern<<<grid, kThreads, smem, st>>>(imga, imgb, albedo, normal, vara, varb, sda, sdb, beta, chol, cond_limit, fallbacks, H, W, hw, sp);
         return cudaGetLastError();
     };
     if (!fixed_rows(hw, sp)) return go(regression_kernel<0>, regression_geom<0>(hw, sp));
@@ -864,9 +870,8 @@ cudaError_t launch_recon(const float *imga, const float *imgb, const float *albe
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         dim3 block(kRX, kRThreadRows), grid((Wr + kRX - 1) / kRX, (Hr + rows - 1) / rows, B);
-        kern<<<grid, block, smem, st>>>(imga, imgb, albedo, normal, vara, varb, sda, sdb, beta, outa, outb, state, H,
-                                        W, hw, sp, rs);
-        return cudaGetLastError();
+        return launch_chained(kern, grid, block, smem, st, imga, imgb, albedo, normal, vara, varb, sda, sdb, beta,
+                              outa, outb, state, H, W, hw, sp, rs);
     };
     return recon_smem(hw, sp, rs, 2 * kRThreadRows) <= kReconPairSmem ? go(recon_kernel<2>, 2)
                                                                       : go(recon_kernel<1>, 1);

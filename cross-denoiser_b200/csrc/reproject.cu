@@ -20,6 +20,7 @@
 // travels by value in the kernel parameters.
 #include <cuda_runtime.h>
 #include "cd_common.cuh"
+#include "launch.cuh"
 
 namespace cd {
 namespace {
@@ -67,6 +68,8 @@ __global__ void __launch_bounds__(256) reproject_kernel(
     const float *__restrict__ opac, const float *__restrict__ popac,
     uint8_t *__restrict__ success, int H, int W)
 {
+    chain_wait();
+    chain_next();
     const int cx = blockIdx.x * blockDim.x + threadIdx.x;
     const int cy = blockIdx.y * blockDim.y + threadIdx.y;
     if (cx >= W || cy >= H) return;
@@ -228,6 +231,8 @@ __global__ void __launch_bounds__(256) reproject_decide_kernel(
     const float *__restrict__ nrm, const float *__restrict__ pnrm, const float *__restrict__ pnfw,
     const float *__restrict__ opac, const float *__restrict__ popac, uint8_t *__restrict__ success, int H, int W)
 {
+    chain_wait();
+    chain_next();
     const int cx = blockIdx.x * blockDim.x + threadIdx.x;
     const int cy = blockIdx.y * blockDim.y + threadIdx.y;
     if (cx >= W || cy >= H) return;
@@ -286,6 +291,8 @@ __global__ void __launch_bounds__(256) reproject_gather_kernel(
     const float *__restrict__ plinz, const float *__restrict__ nrm, const float *__restrict__ pnrm,
     const float *__restrict__ pnfw, const float *__restrict__ popac, uint8_t *__restrict__ success, int H, int W)
 {
+    chain_wait();
+    chain_next();
     const int cx = blockIdx.x * blockDim.x + threadIdx.x;
     const int cy = blockIdx.y * blockDim.y + threadIdx.y;
     if (cx >= W || cy >= H) return;
@@ -368,15 +375,14 @@ cudaError_t launch_reproject(const float *mvec, const ReprojectList &list, const
     bool fast = list.n == 3;
     for (int d = 0; d < list.n; ++d) fast = fast && list.ch[d] == 3;
     if (fast) {
-        reproject_decide_kernel<<<grid, block, 0, st>>>(mvec, linz, plinz, nrm, pnrm, pnfw, opac, popac, success,
-                                                        H, W);
-        reproject_gather_kernel<<<grid, block, 0, st>>>(mvec, list, linz, plinz, nrm, pnrm, pnfw, popac, success, H,
-                                                        W);
+        const cudaError_t e = launch_chained(reproject_decide_kernel, grid, block, 0, st, mvec, linz, plinz, nrm, pnrm,
+                                             pnfw, opac, popac, success, H, W);
+        if (e != cudaSuccess) return e;
+        return launch_chained(reproject_gather_kernel, grid, block, 0, st, mvec, list, linz, plinz, nrm, pnrm, pnfw,
+                              popac, success, H, W);
     }
-    else
-        reproject_kernel<0, 0><<<grid, block, 0, st>>>(mvec, list, linz, plinz, nrm, pnrm, pnfw,
-                                                       opac, popac, success, H, W);
-    return cudaGetLastError();
+    return launch_chained(reproject_kernel<0, 0>, grid, block, 0, st, mvec, list, linz, plinz, nrm, pnrm, pnfw, opac,
+                          popac, success, H, W);
 }
 
 }  // namespace cd

@@ -19,6 +19,7 @@
 // unrolled, other radii take the radius at run time.
 #include <cuda_runtime.h>
 #include "cd_common.cuh"
+#include "launch.cuh"
 #include "filter_sweep.cuh"
 
 namespace cd {
@@ -33,6 +34,8 @@ __global__ void __launch_bounds__(256) sf_forward_kernel(
     const float *__restrict__ band, float *__restrict__ acca, float *__restrict__ accb,
     float *__restrict__ wsa, float *__restrict__ wsb, int H, int W, int hw_rt)
 {
+    chain_wait();
+    chain_next();
     extern __shared__ ulonglong2 tile[];
     const int hw = HW > 0 ? HW : hw_rt;
     const int tw = fsw::kBX + 2 * hw, th = fsw::kBY + 2 * hw;
@@ -62,6 +65,8 @@ __global__ void __launch_bounds__(256, 3) sf_grad_kernel(
     const float *__restrict__ albedo, const float *__restrict__ normal,
     const float *__restrict__ band, float *__restrict__ gband, int H, int W, int hw_rt)
 {
+    chain_wait();
+    chain_next();
     extern __shared__ ulonglong2 tile[];
     const int hw = HW > 0 ? HW : hw_rt;
     const int tw = fsw::kBX + 2 * hw, th = fsw::kBY + 2 * hw;
@@ -95,6 +100,8 @@ __global__ void __launch_bounds__(256) sf_forward_store_kernel(
     const float *__restrict__ band, float *__restrict__ acca, float *__restrict__ accb,
     float *__restrict__ wsa, float *__restrict__ wsb, float4 *__restrict__ part, int H, int W, int hw_rt)
 {
+    chain_wait();
+    chain_next();
     extern __shared__ ulonglong2 tile[];
     const int hw = HW > 0 ? HW : hw_rt;
     const int tw = fsw::kBX + 2 * hw, th = fsw::kBY + 2 * hw;
@@ -128,6 +135,8 @@ __global__ void __launch_bounds__(256) sf_grad_stored_kernel(const float *__rest
                                                              const float4 *__restrict__ part,
                                                              float *__restrict__ gband, size_t n)
 {
+    chain_wait();
+    chain_next();
     const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     fsw::Sums s;
@@ -170,9 +179,8 @@ cudaError_t launch_spatial_filter_store(const float *imga, const float *imgb, co
         cudaError_t e = cudaFuncSetAttribute(sf_forward_store_kernel<R>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        sf_forward_store_kernel<R><<<grid, block, smem, st>>>(imga, imgb, albedo, normal, band, acca, accb, wsa,
-                                                              wsb, reinterpret_cast<float4 *>(partials), H, W, hw);
-        return cudaGetLastError();
+        return launch_chained(sf_forward_store_kernel<R>, grid, block, smem, st, imga, imgb, albedo, normal, band,
+                              acca, accb, wsa, wsb, reinterpret_cast<float4 *>(partials), H, W, hw);
     });
 }
 
@@ -181,9 +189,8 @@ cudaError_t launch_spatial_filter_grad_stored(const float *gacca, const float *g
                                               int W, cudaStream_t st)
 {
     const size_t n = (size_t)B * H * W;
-    sf_grad_stored_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(
-        gacca, gaccb, gwsa, gwsb, reinterpret_cast<const float4 *>(partials), gband, n);
-    return cudaGetLastError();
+    return launch_chained(sf_grad_stored_kernel, (unsigned)((n + 255) / 256), 256, 0, st, gacca, gaccb, gwsa, gwsb,
+                          reinterpret_cast<const float4 *>(partials), gband, n);
 }
 
 cudaError_t launch_spatial_filter(const float *imga, const float *imgb, const float *albedo,
@@ -199,9 +206,8 @@ cudaError_t launch_spatial_filter(const float *imga, const float *imgb, const fl
         cudaError_t e = cudaFuncSetAttribute(sf_forward_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return e;
-        sf_forward_kernel<R><<<grid, block, smem, st>>>(imga, imgb, albedo, normal, band, acca, accb, wsa, wsb,
-                                                        H, W, hw);
-        return cudaGetLastError();
+        return launch_chained(sf_forward_kernel<R>, grid, block, smem, st, imga, imgb, albedo, normal, band, acca,
+                              accb, wsa, wsb, H, W, hw);
     });
 }
 
@@ -219,9 +225,8 @@ cudaError_t launch_spatial_filter_grad(const float *gacca, const float *gaccb, c
         cudaError_t e = cudaFuncSetAttribute(sf_grad_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
         if (e != cudaSuccess) return e;
-        sf_grad_kernel<R><<<grid, block, smem, st>>>(gacca, gaccb, gwsa, gwsb, imga, imgb, albedo, normal, band,
-                                                     gband, H, W, hw);
-        return cudaGetLastError();
+        return launch_chained(sf_grad_kernel<R>, grid, block, smem, st, gacca, gaccb, gwsa, gwsb, imga, imgb, albedo,
+                              normal, band, gband, H, W, hw);
     });
 }
 

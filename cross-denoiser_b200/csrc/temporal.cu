@@ -28,6 +28,7 @@
 #include <atomic>
 #include <cuda_runtime.h>
 #include "cd_common.cuh"
+#include "launch.cuh"
 #include "tma.cuh"
 
 namespace cd {
@@ -59,6 +60,8 @@ CD_DEV float eroded_at(const uint8_t *mask, int x, int y, int H, int W)
 __global__ void __launch_bounds__(256) erode_kernel(const uint8_t *__restrict__ mask,
                                                     float *__restrict__ out, int H, int W)
 {
+    chain_wait();
+    chain_next();
     const int x = blockIdx.x * blockDim.x + threadIdx.x;
     const int y = blockIdx.y * blockDim.y + threadIdx.y;
     if (x >= W || y >= H) return;
@@ -75,6 +78,8 @@ __global__ void __launch_bounds__(kTX * kTY, 3) temporal_kernel(
     float *__restrict__ out1, float *__restrict__ out2, float *__restrict__ succ, int H, int W,
     int hc, int hp)
 {
+    chain_wait();
+    chain_next();
     extern __shared__ float sm[];
     const int tw = kTX + 2 * hc, th = kTY + 2 * hc;
     const int tplane = tw * th, rplane = th * kTX;
@@ -315,6 +320,8 @@ __global__ void __launch_bounds__(kTX * kTY, 2) temporal_tma_kernel(
     float *__restrict__ out1, float *__restrict__ out2, float *__restrict__ succ, int H, int W, int ntx,
     int nty, int ntiles)
 {
+    chain_wait();
+    chain_next();
     using G = TsGeom<HC>;
     extern __shared__ __align__(128) unsigned char smem[];
     float *rmin = reinterpret_cast<float *>(smem + 2 * G::STAGE);
@@ -509,10 +516,9 @@ cudaError_t launch_temporal_tma(const float *c1, const float *c2, const float *p
     }
     const int ntx = (W + kTX - 1) / kTX, nty = (H + kTY - 1) / kTY, ntiles = ntx * nty * B;
     const int grid = min(ntiles, nsm * occ);
-    temporal_tma_kernel<HC><<<grid, dim3(kTX, kTY), G::SMEM, st>>>(m, eroded, out, out1, out2, succ, H, W, ntx, nty,
-                                                                   ntiles);
     *done = true;
-    return cudaGetLastError();
+    return launch_chained(temporal_tma_kernel<HC>, grid, dim3(kTX, kTY), G::SMEM, st, m, eroded, out, out1, out2,
+                          succ, H, W, ntx, nty, ntiles);
 }
 
 }  // namespace
@@ -528,8 +534,7 @@ cudaError_t launch_erode3x3(const uint8_t *mask, float *out, int B, int H, int W
 {
     dim3 block(32, 8);
     dim3 grid((W + 31) / 32, (H + 7) / 8, B);
-    erode_kernel<<<grid, block, 0, st>>>(mask, out, H, W);
-    return cudaGetLastError();
+    return launch_chained(erode_kernel, grid, block, 0, st, mask, out, H, W);
 }
 
 cudaError_t launch_temporal(const float *c1, const float *c2, const float *prev,
@@ -558,16 +563,15 @@ cudaError_t launch_temporal(const float *c1, const float *c2, const float *prev,
         e = cudaFuncSetAttribute(temporal_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem);
         if (e != cudaSuccess) return e;
-        temporal_kernel<true><<<grid, block, smem, st>>>(c1, c2, prev, prev1, prev2, nullptr, raw,
-                                                         eroded, out, out1, out2, succ, H, W, hc, hp);
+        return launch_chained(temporal_kernel<true>, grid, block, smem, st, c1, c2, prev, prev1, prev2, nullptr, raw,
+                             eroded, out, out1, out2, succ, H, W, hc, hp);
     } else {
         e = cudaFuncSetAttribute(temporal_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem);
         if (e != cudaSuccess) return e;
-        temporal_kernel<false><<<grid, block, smem, st>>>(c1, c2, prev, prev1, prev2, rs, nullptr,
-                                                          nullptr, out, out1, out2, succ, H, W, hc, hp);
+        return launch_chained(temporal_kernel<false>, grid, block, smem, st, c1, c2, prev, prev1, prev2, rs, nullptr,
+                             nullptr, out, out1, out2, succ, H, W, hc, hp);
     }
-    return cudaGetLastError();
 }
 
 }  // namespace cd
