@@ -10,13 +10,13 @@ once per frame.
 """
 from __future__ import annotations
 
-import ctypes
 from typing import List, Tuple
 
 import numpy as np
 import torch
 
 from . import _lib
+from .ops import _ptr, _stream
 
 LEARNING_RATE = 1e-3        # scripts/main.py:74
 BETA1, BETA2, EPSILON = 0.9, 0.999, 1e-7   # keras.optimizers.Adam defaults
@@ -73,14 +73,6 @@ def split_params(flat) -> list:
         out.append(flat[o:o + n].reshape(shape))
         o += n
     return out
-
-
-def _ptr(t):
-    return ctypes.c_void_p(t.data_ptr())
-
-
-def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 class UNet:
