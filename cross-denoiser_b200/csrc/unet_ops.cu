@@ -36,14 +36,15 @@ CD_DEV void ld8(const __nv_bfloat16 *p, float *v)
         v[2 * e + 1] = f.y;
     }
 }
-CD_DEV void st8(__nv_bfloat16 *p, const float *v)
+CD_DEV uint4 pack8(const float *v)
 {
     uint4 o;
     __nv_bfloat162 *h = reinterpret_cast<__nv_bfloat162 *>(&o);
 #pragma unroll
     for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
-    *reinterpret_cast<uint4 *>(p) = o;
+    return o;
 }
+CD_DEV void st8(__nv_bfloat16 *p, const float *v) { *reinterpret_cast<uint4 *>(p) = pack8(v); }
 
 // [ols1, ols2, prev_out, albedo, normal] (fp32, 3 channels each) -> bf16, 16
 // channels (15 + zero) in two row-chunk planes; n = B * H * W pixels, W wide
@@ -70,11 +71,15 @@ __global__ void __launch_bounds__(256) pack_input_kernel(const float *__restrict
     st8(x + act_idx(0, row, 1, px, 0, W, 2) * 8, v + 8);
 }
 
-// Conv2DTranspose(kernel 1, stride 2) forward, one thread per input pixel
-// (i, j): output (2i, 2j) = K x + b (each channel summed over ci in order,
-// K rows read as float4), outputs (2i, 2j + 1), (2i + 1, 2j), (2i + 1, 2j + 1)
-// = b.
-template <int CI, int CO>
+// Conv2DTranspose(kernel 1, stride 2) forward: output (2i, 2j) = K x + b
+// (each channel summed over ci in order, K rows read as float4), outputs
+// (2i, 2j + 1), (2i + 1, 2j), (2i + 1, 2j + 1) = b.  A weight read from
+// shared memory costs its 128 bytes per warp whatever the lanes share, and
+// with one pixel per thread those reads bound the kernel, so a thread takes
+// kPix input pixels (a block apart) per weight, and lanes trade pixels so that
+// every store is 512 consecutive bytes: 32 channels at 480x270 22 -> 16 us, 16
+// at 960x540 27 -> 18.
+template <int CI, int CO, int kPix>
 __global__ void __launch_bounds__(256) tconv_fwd_kernel(const __nv_bfloat16 *__restrict__ in,
                                                         const float *__restrict__ K, const float *__restrict__ bias,
                                                         __nv_bfloat16 *__restrict__ out, int Hi, int Wi, int B)
@@ -85,34 +90,62 @@ __global__ void __launch_bounds__(256) tconv_fwd_kernel(const __nv_bfloat16 *__r
     for (int i = threadIdx.x; i < CO * CI + CO; i += blockDim.x) sK[i] = i < CO * CI ? K[i] : bias[i - CO * CI];
     __syncthreads();
     const int Ho = 2 * Hi, Wo = 2 * Wi;
-    const size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= (size_t)B * Hi * Wi) return;
-    const int xi = (int)(p % Wi), yi = (int)((p / Wi) % Hi), b = (int)(p / ((size_t)Wi * Hi));
-    float x[CI];
+    const size_t n = (size_t)B * Hi * Wi, p0 = (size_t)blockIdx.x * blockDim.x * kPix + threadIdx.x;
+    float x[kPix][CI];
+    unsigned at[kPix];   // output (2i, 2j), chunk 0, in 8-channel units; kNone past the last pixel
+    constexpr unsigned kNone = 0xFFFFFFFFu;
 #pragma unroll
-    for (int c = 0; c < CI; c += 8) ld8(in + act_idx(b, yi, c / 8, xi, Hi, Wi, CI / 8) * 8, x + c);
-    float o[CO], ob[CO];
+    for (int k = 0; k < kPix; ++k) {
+        const size_t p = p0 + (size_t)k * blockDim.x, q = p < n ? p : 0;
+        const int xi = (int)(q % Wi), yi = (int)((q / Wi) % Hi), b = (int)(q / ((size_t)Wi * Hi));
+        at[k] = p < n ? (unsigned)act_idx(b, 2 * yi, 0, 2 * xi, Ho, Wo, CO / 8) : kNone;
 #pragma unroll
-    for (int co = 0; co < CO; ++co) {
-        ob[co] = sK[CO * CI + co];
-        float s = ob[co];
-        const float4 *kr = reinterpret_cast<const float4 *>(sK + co * CI);
-#pragma unroll
-        for (int c4 = 0; c4 < CI / 4; ++c4) {
-            const float4 k4 = kr[c4];
-            s = fmaf(k4.x, x[4 * c4], s);
-            s = fmaf(k4.y, x[4 * c4 + 1], s);
-            s = fmaf(k4.z, x[4 * c4 + 2], s);
-            s = fmaf(k4.w, x[4 * c4 + 3], s);
-        }
-        o[co] = s;
+        for (int c = 0; c < CI; c += 8) ld8(in + act_idx(b, yi, c / 8, xi, Hi, Wi, CI / 8) * 8, x[k] + c);
     }
-#pragma unroll
+    const int lane = threadIdx.x & 31;
+    uint4 *out4 = reinterpret_cast<uint4 *>(out);
+#pragma unroll 1
     for (int c = 0; c < CO; c += 8) {
-        st8(out + act_idx(b, 2 * yi, c / 8, 2 * xi, Ho, Wo, CO / 8) * 8, o + c);
-        st8(out + act_idx(b, 2 * yi, c / 8, 2 * xi + 1, Ho, Wo, CO / 8) * 8, ob + c);
-        st8(out + act_idx(b, 2 * yi + 1, c / 8, 2 * xi, Ho, Wo, CO / 8) * 8, ob + c);
-        st8(out + act_idx(b, 2 * yi + 1, c / 8, 2 * xi + 1, Ho, Wo, CO / 8) * 8, ob + c);
+        float o[kPix][8], ob[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            ob[e] = sK[CO * CI + c + e];
+#pragma unroll
+            for (int k = 0; k < kPix; ++k) o[k][e] = ob[e];
+            const float4 *kr = reinterpret_cast<const float4 *>(sK + (c + e) * CI);
+#pragma unroll
+            for (int c4 = 0; c4 < CI / 4; ++c4) {
+                const float4 k4 = kr[c4];
+#pragma unroll
+                for (int k = 0; k < kPix; ++k) {
+                    float t = fmaf(k4.x, x[k][4 * c4], o[k][e]);
+                    t = fmaf(k4.y, x[k][4 * c4 + 1], t);
+                    t = fmaf(k4.z, x[k][4 * c4 + 2], t);
+                    o[k][e] = fmaf(k4.w, x[k][4 * c4 + 3], t);
+                }
+            }
+        }
+        const uint4 vb = pack8(ob);
+#pragma unroll
+        for (int k = 0; k < kPix; ++k) {
+            // the warp's 64 output pixels of each row, 32 consecutive ones per
+            // store: lane l takes pixel 32 j + l, input pixel (32 j + l) / 2's
+            const uint4 v = pack8(o[k]);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int src = 16 * j + (lane >> 1);
+                const unsigned base = __shfl_sync(0xffffffffu, at[k], src);
+                uint4 t;
+                t.x = __shfl_sync(0xffffffffu, v.x, src);
+                t.y = __shfl_sync(0xffffffffu, v.y, src);
+                t.z = __shfl_sync(0xffffffffu, v.z, src);
+                t.w = __shfl_sync(0xffffffffu, v.w, src);
+                if (base == kNone) continue;
+                const size_t i = (size_t)base + (size_t)(c / 8) * Wo + (lane & 1);
+                out4[i] = lane & 1 ? vb : t;
+                out4[i + (size_t)(CO / 8) * Wo] = vb;
+            }
+        }
     }
 }
 
@@ -250,108 +283,208 @@ __global__ void __launch_bounds__(kN) tconv_bwd_kernel(const __nv_bfloat16 *__re
 }
 
 // Head: param = Kh^T c5_1 + bh (Kh[ci][co], 8 x 6), band = 1 / (p^2 + 1e-4), alpha = sigmoid(p5).
-// A block's band values (five per pixel) go out through shared memory as
-// float4 stores.
-__global__ void __launch_bounds__(256) head_fwd_kernel(const __nv_bfloat16 *__restrict__ x, const float *__restrict__ K,
-                                                       const float *__restrict__ bias, float *__restrict__ band,
-                                                       float *__restrict__ alpha, size_t n)
+// A thread takes two pixels per weight read (as tconv_fwd_kernel), 256
+// apart; a block's band values (five per pixel) go out through shared
+// memory as float4 stores.  2560x1440: 41 -> 32 us.
+constexpr int kHeadThreads = 256;
+
+// param co of a pixel's v, weights sT[co][ci] (co = 0..5), summed over ci in order
+CD_DEV void head_params(const float4 *sT, const float *bias, const float (&v)[2][8], float (&q)[2][6])
+{
+#pragma unroll
+    for (int co = 0; co < 6; ++co) {
+        const float4 k0 = sT[2 * co], k1 = sT[2 * co + 1];
+        const float kk[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w}, bc = bias[co];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            float t = bc;
+#pragma unroll
+            for (int ci = 0; ci < 8; ++ci) t = fmaf(kk[ci], v[i][ci], t);
+            q[i][co] = t;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kHeadThreads) head_fwd_kernel(const __nv_bfloat16 *__restrict__ x,
+                                                                const float *__restrict__ K,
+                                                                const float *__restrict__ bias,
+                                                                float *__restrict__ band, float *__restrict__ alpha,
+                                                                size_t n)
 {
     chain_wait();
     chain_next();
-    __shared__ float sK[54];
-    __shared__ __align__(16) float sb[256 * 5];   // the block's band values, written out as float4
+    __shared__ __align__(16) float sT[48];
+    __shared__ float sB[6];
+    __shared__ __align__(16) float sb[2 * kHeadThreads * 5];   // the block's band values, written out as float4
     const int tid = threadIdx.x;
-    if (tid < 54) sK[tid] = tid < 48 ? K[tid] : bias[tid - 48];
+    const size_t p0 = (size_t)blockIdx.x * (2 * kHeadThreads);
+    float v[2][8];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const size_t p = p0 + i * kHeadThreads + tid;
+        ld8(x + 8 * (p < n ? p : 0), v[i]);
+    }
+    if (tid < 48) sT[(tid % 6) * 8 + tid / 6] = K[tid];
+    if (tid < 6) sB[tid] = bias[tid];
     __syncthreads();
-    const size_t p0 = (size_t)blockIdx.x * 256, p = p0 + tid;
-    if (p < n) {
-        float v[8];
-        ld8(x + 8 * p, v);
-        float q[6];
+    float q[2][6];
+    head_params(reinterpret_cast<const float4 *>(sT), sB, v, q);
 #pragma unroll
-        for (int co = 0; co < 6; ++co) {
-            float s = sK[48 + co];
+    for (int i = 0; i < 2; ++i) {
+        const int t = i * kHeadThreads + tid;
 #pragma unroll
-            for (int ci = 0; ci < 8; ++ci) s = fmaf(sK[ci * 6 + co], v[ci], s);
-            q[co] = s;
-        }
-#pragma unroll
-        for (int k = 0; k < 5; ++k) sb[5 * tid + k] = 1.f / (q[k] * q[k] + 1e-4f);
-        alpha[p] = 1.f / (1.f + expf(-q[5]));
+        for (int k = 0; k < 5; ++k) sb[5 * t + k] = 1.f / (q[i][k] * q[i][k] + 1e-4f);
+        if (p0 + t < n) alpha[p0 + t] = 1.f / (1.f + expf(-q[i][5]));
     }
     __syncthreads();
-    const int cnt = 5 * (int)(n - p0 < 256 ? n - p0 : 256);
+    const int cnt = 5 * (int)(n - p0 < 2 * kHeadThreads ? n - p0 : 2 * kHeadThreads);
     float *dst = band + 5 * p0;
     int i = tid;
     if (!(reinterpret_cast<uintptr_t>(dst) & 15)) {
-        for (; i < cnt / 4; i += 256) reinterpret_cast<float4 *>(dst)[i] = reinterpret_cast<const float4 *>(sb)[i];
+        for (; i < cnt / 4; i += kHeadThreads)
+            reinterpret_cast<float4 *>(dst)[i] = reinterpret_cast<const float4 *>(sb)[i];
         i = (cnt / 4) * 4 + tid;
     }
-    for (; i < cnt; i += 256) dst[i] = sb[i];
+    for (; i < cnt; i += kHeadThreads) dst[i] = sb[i];
 }
 
 // Head backward: dZ of c5_1 (times its ReLU derivative) and the block's
 // partial sums of dKh[ci][co] and dbh[co].  Each thread walks pixels
 // p = thread, thread + grid size, ... accumulating its 54 parameter-gradient
-// terms in registers; the block then reduces them (lanes, then warps, in a
-// fixed order) to one partial row.
-constexpr int kHeadThreads = 256;
+// terms in registers (in that order); the block then reduces them (lanes,
+// then warps, in a fixed order) to one partial row.
+//
+// 128 registers leave two blocks an SM, too few loads in flight to cover
+// DRAM from registers: every warp copies its pixels' inputs (32 activations,
+// band and alpha gradients) kHeadAhead iterations ahead into slots of its
+// own (cp.async, no block barrier).  Two iterations at a time share the weight
+// reads.  2560x1440: 98 -> 60 us.
 constexpr int kHeadMaxBlocks = 592;
+constexpr int kHeadAhead = 4, kHeadSlots = kHeadAhead + 2;
+struct __align__(16) HeadSlot {
+    uint4 x[32];
+    float gband[160], galpha[32];
+};
+constexpr int kHeadBwdSmem = kHeadSlots * (kHeadThreads / 32) * (int)sizeof(HeadSlot);
 
-__global__ void __launch_bounds__(kHeadThreads) head_bwd_kernel(const __nv_bfloat16 *__restrict__ x,
-                                                                const float *__restrict__ K,
-                                                                const float *__restrict__ bias,
-                                                                const float *__restrict__ gband,
-                                                                const float *__restrict__ galpha,
-                                                                __nv_bfloat16 *__restrict__ dz,
-                                                                float *__restrict__ partial, size_t n)
+CD_DEV void head_cp(void *dst, const void *src, int bytes)   // bytes: 4 or 16
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    if (bytes == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+    else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+}
+
+__global__ void __launch_bounds__(kHeadThreads, 2) head_bwd_kernel(const __nv_bfloat16 *__restrict__ x,
+                                                                   const float *__restrict__ K,
+                                                                   const float *__restrict__ bias,
+                                                                   const float *__restrict__ gband,
+                                                                   const float *__restrict__ galpha,
+                                                                   __nv_bfloat16 *__restrict__ dz,
+                                                                   float *__restrict__ partial, size_t n)
 {
     chain_wait();
     chain_next();
-    __shared__ float sK[54];
+    extern __shared__ __align__(16) uint8_t head_smem[];
+    __shared__ __align__(16) float sK[48], sT[48];   // Kh[ci][co], and transposed
+    __shared__ float sB[6];
     __shared__ float red[kHeadThreads / 32][54];
-    const int tid = threadIdx.x;
-    if (tid < 54) sK[tid] = tid < 48 ? K[tid] : bias[tid - 48];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    HeadSlot *slots = reinterpret_cast<HeadSlot *>(head_smem) + warp * kHeadSlots;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(gband) | reinterpret_cast<uintptr_t>(galpha)) & 15) == 0;
+    const size_t w0 = (size_t)blockIdx.x * kHeadThreads + warp * 32, step = (size_t)gridDim.x * kHeadThreads;
+    auto fetch = [&](int k) {   // iteration k's inputs, one group
+        const size_t p = w0 + k * step;
+        HeadSlot &s = slots[k % kHeadSlots];
+        if (p + 32 <= n && aligned) {
+            head_cp(&s.x[lane], x + 8 * (p + lane), 16);
+            head_cp(&s.gband[4 * lane], gband + 5 * p + 4 * lane, 16);
+            if (lane < 8) {
+                head_cp(&s.gband[128 + 4 * lane], gband + 5 * p + 128 + 4 * lane, 16);
+                head_cp(&s.galpha[4 * lane], galpha + p + 4 * lane, 16);
+            }
+        } else if (p + lane < n) {
+            head_cp(&s.x[lane], x + 8 * (p + lane), 16);
+#pragma unroll
+            for (int e = 0; e < 5; ++e) head_cp(&s.gband[5 * lane + e], gband + 5 * (p + lane) + e, 4);
+            head_cp(&s.galpha[lane], galpha + p + lane, 4);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll
+    for (int k = 0; k < kHeadAhead; ++k) fetch(k);
+    if (tid < 48) {
+        const float w = K[tid];
+        sK[tid] = w;
+        sT[(tid % 6) * 8 + tid / 6] = w;
+    }
+    if (tid < 6) sB[tid] = bias[tid];
     __syncthreads();
-    const int lane = tid & 31, warp = tid >> 5;
     float acc[54];
 #pragma unroll
     for (int j = 0; j < 54; ++j) acc[j] = 0.f;
-    for (size_t p = (size_t)blockIdx.x * kHeadThreads + tid; p < n; p += (size_t)gridDim.x * kHeadThreads) {
-        float v[8], g[6];
-        ld8(x + 8 * p, v);
+    for (int k = 0; w0 + k * step < n; k += 2) {
+        fetch(k + kHeadAhead);
+        fetch(k + kHeadAhead + 1);
+        asm volatile("cp.async.wait_group %0;" ::"n"(kHeadAhead) : "memory");
+        __syncwarp();
+        float v[2][8], g[2][6], d[2][8];
+        bool in[2];
 #pragma unroll
-        for (int co = 0; co < 6; ++co) {
-            float s = sK[48 + co];
+        for (int i = 0; i < 2; ++i) {
+            const HeadSlot &s = slots[(k + i) % kHeadSlots];
+            in[i] = w0 + (k + i) * step + lane < n;
+            ld8(reinterpret_cast<const __nv_bfloat16 *>(&s.x[lane]), v[i]);
 #pragma unroll
-            for (int ci = 0; ci < 8; ++ci) s = fmaf(sK[ci * 6 + co], v[ci], s);
-            if (co < 5) {
-                // d band / d s = -2 s / (s^2 + 1e-4)^2, with one fast
-                // reciprocal (a gradient: FP32 tolerance, not the forward's
-                // rounding)
-                const float r = __fdividef(1.f, s * s + 1e-4f);
-                g[co] = __ldg(gband + 5 * p + co) * (-2.f * s * r * r);
-            } else {
-                const float a = 1.f / (1.f + expf(-s));
-                g[co] = __ldg(galpha + p) * a * (1.f - a);
+            for (int e = 0; e < 5; ++e) g[i][e] = s.gband[5 * lane + e];
+            g[i][5] = s.galpha[lane];
+        }
+        float q[2][6];
+        head_params(reinterpret_cast<const float4 *>(sT), sB, v, q);
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int co = 0; co < 6; ++co) {
+                const float t = q[i][co];
+                if (co < 5) {
+                    // d band / d t = -2 t / (t^2 + 1e-4)^2, with one fast
+                    // reciprocal (a gradient: FP32 tolerance, not the forward's
+                    // rounding)
+                    const float r = __fdividef(1.f, t * t + 1e-4f);
+                    g[i][co] = g[i][co] * (-2.f * t * r * r);
+                } else {
+                    const float a = 1.f / (1.f + expf(-t));
+                    g[i][co] = g[i][co] * a * (1.f - a);
+                }
             }
+#pragma unroll
+        for (int ci = 0; ci < 8; ci += 2) {   // two rows of Kh: twelve weights
+            const float4 *kr = reinterpret_cast<const float4 *>(sK + 6 * ci);
+            const float4 k0 = kr[0], k1 = kr[1], k2 = kr[2];
+            const float kk[12] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w, k2.x, k2.y, k2.z, k2.w};
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    float t = 0.f;
+#pragma unroll
+                    for (int co = 0; co < 6; ++co) t = fmaf(kk[6 * c + co], g[i][co], t);
+                    d[i][ci + c] = v[i][ci + c] > 0.f ? t : 0.f;
+                }
         }
-        float d[8];
 #pragma unroll
-        for (int ci = 0; ci < 8; ++ci) {
-            float s = 0.f;
+        for (int i = 0; i < 2; ++i)
+            if (in[i]) {
+                st8(dz + 8 * (w0 + (k + i) * step + lane), d[i]);
 #pragma unroll
-            for (int co = 0; co < 6; ++co) s = fmaf(sK[ci * 6 + co], g[co], s);
-            d[ci] = v[ci] > 0.f ? s : 0.f;
-        }
-        st8(dz + 8 * p, d);
+                for (int ci = 0; ci < 8; ++ci)
 #pragma unroll
-        for (int ci = 0; ci < 8; ++ci)
+                    for (int co = 0; co < 6; ++co) acc[ci * 6 + co] = fmaf(v[i][ci], g[i][co], acc[ci * 6 + co]);
 #pragma unroll
-            for (int co = 0; co < 6; ++co) acc[ci * 6 + co] = fmaf(v[ci], g[co], acc[ci * 6 + co]);
-#pragma unroll
-        for (int co = 0; co < 6; ++co) acc[48 + co] += g[co];
+                for (int co = 0; co < 6; ++co) acc[48 + co] += g[i][co];
+            }
+        __syncwarp();   // both slots are read before a later fetch writes them
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
     for (int j = 0; j < 54; ++j) {
         float s = acc[j];
@@ -490,11 +623,12 @@ cudaError_t launch_tconv_fwd(int ci, int co, const __nv_bfloat16 *in, const floa
                              __nv_bfloat16 *out, int Hi, int Wi, int B, cudaStream_t st)
 {
     const size_t n = (size_t)B * Hi * Wi;
-    const unsigned g = (unsigned)((n + 255) / 256);
-    if (ci == 32 && co == 32) return launch_chained(tconv_fwd_kernel<32, 32>, g, 256, 0, st, in, K, bias, out, Hi,
-                                                    Wi, B);
-    if (ci == 16 && co == 16) return launch_chained(tconv_fwd_kernel<16, 16>, g, 256, 0, st, in, K, bias, out, Hi,
-                                                    Wi, B);
+    auto go = [&](auto kern, int threads, int pix) {
+        return launch_chained(kern, (unsigned)((n + threads * pix - 1) / (threads * pix)), threads, 0, st, in, K, bias,
+                              out, Hi, Wi, B);
+    };
+    if (ci == 32 && co == 32) return go(tconv_fwd_kernel<32, 32, 2>, 64, 2);
+    if (ci == 16 && co == 16) return go(tconv_fwd_kernel<16, 16, 2>, 128, 2);
     return cudaErrorInvalidValue;
 }
 
@@ -525,7 +659,8 @@ cudaError_t launch_tconv_bwd(int ci, int co, const __nv_bfloat16 *in, const __nv
 cudaError_t launch_head_fwd(const __nv_bfloat16 *x, const float *K, const float *bias, float *band, float *alpha,
                             size_t n, cudaStream_t st)
 {
-    return launch_chained(head_fwd_kernel, (unsigned)((n + 255) / 256), 256, 0, st, x, K, bias, band, alpha, n);
+    return launch_chained(head_fwd_kernel, (unsigned)((n + 2 * kHeadThreads - 1) / (2 * kHeadThreads)), kHeadThreads, 0,
+                          st, x, K, bias, band, alpha, n);
 }
 
 size_t head_blocks(size_t n)
@@ -537,8 +672,10 @@ size_t head_blocks(size_t n)
 cudaError_t launch_head_bwd(const __nv_bfloat16 *x, const float *K, const float *bias, const float *gband,
                             const float *galpha, __nv_bfloat16 *dz, float *partial, size_t n, cudaStream_t st)
 {
-    return launch_chained(head_bwd_kernel, (unsigned)head_blocks(n), kHeadThreads, 0, st, x, K, bias, gband, galpha,
-                          dz, partial, n);
+    cudaError_t e = cudaFuncSetAttribute(head_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHeadBwdSmem);
+    if (e != cudaSuccess) return e;
+    return launch_chained(head_bwd_kernel, (unsigned)head_blocks(n), kHeadThreads, kHeadBwdSmem, st, x, K, bias, gband,
+                          galpha, dz, partial, n);
 }
 
 cudaError_t launch_pool_bwd(int C, const __nv_bfloat16 *act, const __nv_bfloat16 *pooled,

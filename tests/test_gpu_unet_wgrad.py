@@ -50,3 +50,25 @@ def test_network(cd, cuda, B, H, W):
         n = int(np.prod(shape))
         close_to_max(grads[o:o + n], ref[o:o + n], 3e-2, f"param tensor {i} {shape}")
         o += n
+
+
+@pytest.mark.parametrize("B,H,W", [(1, 4, 4), (1, 8, 12), (3, 4, 260), (1, 132, 520)])
+def test_unaligned_gradients(cd, cuda, B, H, W):
+    """Output gradients 4 bytes past a 16-byte boundary take the head
+    backward's 4-byte copies: the same parameter gradients bit for bit, also
+    where the last 32 pixels are not all there."""
+    ins = [t.to(DEV) for t in frame_inputs(B, H, W, H + 7 * W)]
+    g = torch.Generator().manual_seed(W)
+    gb, ga = torch.randn((B, H, W, 5), generator=g).to(DEV), torch.randn((B, H, W, 1), generator=g).to(DEV)
+
+    def shifted(t):
+        v = torch.empty(t.numel() + 1, device=DEV)[1:].view(t.shape)
+        return v.copy_(t)
+
+    net = well_conditioned_net(cd, 3)
+    net(*ins)
+    want = net.backward(gb, ga).clone()
+    got = net.backward(shifted(gb), shifted(ga)).clone()
+    torch.cuda.synchronize()
+    assert net.error_flag() == 0
+    assert torch.equal(got, want)
