@@ -86,7 +86,7 @@ __host__ __device__ inline size_t align1k(size_t n) { return (n + 1023) & ~(size
 __host__ __device__ inline size_t conv_smem(int nsteps, int nout, int c0, int c1, int R)
 {
     return (size_t)b_bytes(nsteps, nout) + align128((size_t)(R + 2) * c0 * kPlane) +
-           align128((size_t)(R + 2) * c1 * kPlane) + 16;
+           align128((size_t)(R + 2) * c1 * kPlane) + 32;
 }
 
 // TMEM columns of a CTA: R row groups of NOUT accumulators, or, ky-stacked,
@@ -211,27 +211,31 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const ConvParams P)
     uint8_t *sA0 = smem + bb;
     uint8_t *sA1 = sA0 + blk0;
     uint64_t *bar = reinterpret_cast<uint64_t *>(sA1 + blk1);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 1);
+    uint64_t *mbar = bar + 1;   // the MMAs' commit
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 2);
 
     // per input source, planes [row][chunk][131 px][8 ch] (zeros outside the
     // image), and the packed weights: bulk copies on one mbarrier
     if (tid == 0) {
-        tc::mbar_init(bar, 1);
+        tc::mbar_init(bar, 4);
+        tc::mbar_init(mbar, 1);
         tc::fence_async_smem();
     }
     chain_wait();
     if (warp == 0) tc::tmem_alloc(tslot, kCols);
-    __syncthreads();   // barrier initialised before the copies are issued and waited on
+    __syncthreads();   // barriers initialised before the copies are issued and waited on
     chain_next();
-    if (warp == 0) {
-        const int lane = tid & 31, nch = P.c0 + P.c1;
+    // every warp issues a quarter of the copies (one warp issues a 2 KB copy
+    // about every 180 cycles)
+    {
+        const int lane = tid & 31, nch = P.c0 + P.c1, nplanes = (R + 2) * nch;
         if (lane == 0) {
-            const uint32_t bytes = (uint32_t)bb + (uint32_t)((R + 2) * nch * kPlane);
-            tc::mbar_expect_tx(bar, bytes);
-            tc::bulk_load(sB, P.wpack, (uint32_t)bb, bar);
+            const uint32_t mine = (uint32_t)((nplanes - warp + 3) / 4 * kPlane);
+            tc::mbar_expect_tx(bar, warp == 0 ? mine + (uint32_t)bb : mine);
+            if (warp == 0) tc::bulk_load(sB, P.wpack, (uint32_t)bb, bar);
         }
-        __syncwarp();   // the transaction count is raised before any copy lands
-        for (int i = lane; i < (R + 2) * nch; i += 32) {
+        __syncwarp();   // the warp's transaction count is raised before its copies land
+        for (int i = warp + 4 * lane; i < nplanes; i += 128) {
             const int r = i / nch, c = i - r * nch, gy = y0 - 1 + r;
             const bool s1 = c >= P.c0;
             const int cs = s1 ? c - P.c0 : c, ns = s1 ? P.c1 : P.c0;
@@ -305,10 +309,9 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const ConvParams P)
                     tc::mma_bf16(tbase + r * NOUT, ad, bd, idesc, s > 0 ? 1u : 0u);
                 }
         }
-        tc::commit(bar);
+        tc::commit(mbar);
     }
-    // the commit completes the barrier's second phase (parity 1)
-    const bool done = __syncthreads_and(tc::mbar_wait(bar, 1, kWaitIter)) != 0;   // uniform across the CTA
+    const bool done = __syncthreads_and(tc::mbar_wait(mbar, 0, kWaitIter)) != 0;   // uniform across the CTA
     tc::fence_after_sync();
     if (!done) {
         if (tid == 0) atomicExch(P.err, 2);
@@ -358,18 +361,21 @@ cudaError_t launch_rows(const ConvParams &P, int B, cudaStream_t st)
 // Persistent, pipelined form of the ky-stacked convolution.  The same MMAs
 // per tile (R output rows x 128 pixels) as conv3x3_kernel<NOUT, R, true>,
 // with the roles split over warps so that staging, tensor-core work and the
-// epilogue of different tiles overlap: warp 0 stages tile i into ring slot
-// i % S (bulk copies; the packed weights once per CTA), lane 0 of warp 1
-// issues the tile's MMAs into TMEM accumulator buffer i % 2 and commits them
-// to the slot's "empty" and the buffer's "full" barriers, and warps 2..5
-// (TMEM lanes = pixels) run the epilogue of the buffer, zero it and hand it
-// back through its "empty" barrier.  The epilogue is the longest of the
+// epilogue of different tiles overlap: two warps stage tile i into ring slot
+// i % S (bulk copies; the packed weights once per CTA), one lane of the next
+// warp issues the tile's MMAs into TMEM accumulator buffer i % 2 and commits
+// them to the slot's "empty" and the buffer's "full" barriers, and the other
+// warps (TMEM lanes = pixels) run the epilogue of the buffer, zero it and hand
+// it back through its "empty" barrier.  The epilogue is the longest of the
 // three per tile, so it has two warps per TMEM lane quadrant, one per pair
 // of output rows (the fused pooling pairs rows 2k, 2k + 1), and two CTAs
-// share an SM where their rings fit half of its shared memory.  Every wait
-// is bounded.
+// share an SM where their rings fit half of its shared memory.  A warp issues
+// a 2 KB bulk copy about every 150 cycles, so two share a tile's copies (and
+// four in the per-tile kernel): the network's prediction at 1920x1080 takes
+// 261 us, with one 266; a third gave nothing.  Every wait is bounded.
+constexpr int kPipeLoadWarps = 2;
 constexpr int kPipeEpiWarps = 8;
-constexpr int kPipeThreads = 64 + 32 * kPipeEpiWarps;
+constexpr int kPipeThreads = 32 * (kPipeLoadWarps + 1 + kPipeEpiWarps);
 constexpr int kPipeSmem = 225 * 1024;     // one CTA per SM
 constexpr int kPipeSmem2 = 112 * 1024;    // two CTAs per SM
 constexpr int kPipeMaxSlots = 8;
@@ -378,7 +384,6 @@ struct ConvPipePlan {
     uint32_t wbytes;   // packed weights (B operand), rounded up to 1 KB
     uint32_t blk0;     // source 0 rows of a slot
     uint32_t stage;    // bytes per ring slot
-    uint32_t tx;       // bytes the copies of one slot deliver
     int S;             // ring slots
     size_t smem;
 };
@@ -389,7 +394,6 @@ inline ConvPipePlan conv_pipe_plan(int nsteps, int nout_rows, int c0, int c1, in
     p.wbytes = (uint32_t)align1k((size_t)b_bytes(nsteps, nout_rows));
     p.blk0 = (uint32_t)align128((size_t)(R + 2) * c0 * kPlane);
     p.stage = (uint32_t)align1k(p.blk0 + align128((size_t)(R + 2) * c1 * kPlane));
-    p.tx = (uint32_t)((R + 2) * (c0 + c1) * kPlane);
     const long room = (long)smem_cap - (long)p.wbytes - 1024;
     const int S = room > 0 ? (int)(room / (long)p.stage) : 0;
     p.S = S > kPipeMaxSlots ? kPipeMaxSlots : S;
@@ -423,10 +427,10 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
     uint32_t *tslot = reinterpret_cast<uint32_t *>(wbar + 1);
 
     chain_wait();
-    if (warp == 1) tc::tmem_alloc(tslot, kCols);
+    if (warp == kPipeLoadWarps) tc::tmem_alloc(tslot, kCols);
     if (tid == 0) {
         for (int s = 0; s < S; ++s) {
-            tc::mbar_init(&full[s], 1);
+            tc::mbar_init(&full[s], kPipeLoadWarps);
             tc::mbar_init(&empty[s], 1);
         }
         for (int k = 0; k < 2; ++k) {
@@ -442,9 +446,10 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
     const uint32_t tbase = *tslot;
     chain_next();
     // both accumulator buffers start at zero (every MMA accumulates)
-    if (warp >= 2) {
+    const int ew = warp - kPipeLoadWarps - 1;   // epilogue warp
+    if (ew >= 0) {
         const uint32_t lanes = tbase + ((uint32_t)((warp & 3) * 32) << 16);
-        const int rp = (warp - 2) >> 2;
+        const int rp = ew >> 2;
         for (int k = 0; k < 2; ++k)
             for (int col = rp * (kGrp / 2); col < (rp + 1) * (kGrp / 2); col += 16)
                 tc::tmem_st16_zero(lanes + (uint32_t)(k * kGrp + col));
@@ -459,15 +464,17 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
     for (int t = first; t < ntiles; t += stride) ++ntile;
     bool ok = true;
 
-    if (warp == 0) {
-        // ---- producer: one bulk copy per chunk plane row (zeros outside
-        // the image), the packed weights once ----
+    if (warp < kPipeLoadWarps) {
+        // ---- producers: one bulk copy per chunk plane row (zeros outside
+        // the image), producer w the planes w, w + kPipeLoadWarps, ...; the
+        // packed weights once ----
         const uint32_t bb = (uint32_t)b_bytes(P.nsteps, kRowsB);
-        if (lane == 0) {
+        if (tid == 0) {
             tc::mbar_expect_tx(wbar, bb);
             tc::bulk_load(sB, P.wpack, bb, wbar);
         }
-        const int nch = P.c0 + P.c1;
+        const int nch = P.c0 + P.c1, nplanes = (R + 2) * nch;
+        const uint32_t my_tx = (uint32_t)((nplanes - warp + kPipeLoadWarps - 1) / kPipeLoadWarps * kPlane);
         int i = 0;
         for (; i < ntile; ++i) {
             const int s = i % S, tile = first + i * stride;
@@ -482,9 +489,9 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
             const int tx = tile % ntx, ty = (tile / ntx) % nty, b = tile / (ntx * nty);
             const int x0 = tx * kPx, y0 = ty * R;
             uint8_t *sA0 = ring + (size_t)s * pl.stage, *sA1 = sA0 + pl.blk0;
-            if (lane == 0) tc::mbar_expect_tx(&full[s], pl.tx);
+            if (lane == 0) tc::mbar_expect_tx(&full[s], my_tx);
             __syncwarp();   // the transaction count is raised before any copy lands
-            for (int q = lane; q < (R + 2) * nch; q += 32) {
+            for (int q = warp + kPipeLoadWarps * lane; q < nplanes; q += 32 * kPipeLoadWarps) {
                 const int r = q / nch, c = q - r * nch, gy = y0 - 1 + r;
                 const bool s1 = c >= P.c0;
                 const int cs = s1 ? c - P.c0 : c, ns = s1 ? P.c1 : P.c0;
@@ -500,7 +507,7 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
             for (int s = 0; s < S && s < i; ++s)
                 tc::mbar_wait(&full[s], (uint32_t)((i - s + S - 1) / S - 1) & 1u, kWaitIter);
         }
-    } else if (warp == 1) {
+    } else if (warp == kPipeLoadWarps) {
         // ---- MMA issue (one thread) ----
         if (lane == 0) {
             const uint32_t idesc = tc::idesc_bf16(kPx, kRowsB);
@@ -545,7 +552,7 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
     } else {
         // ---- epilogue: TMEM lane m = pixel x0 + m, output rows 2 rp, 2 rp + 1 ----
-        const int m = (warp & 3) * 32 + lane, rp = (warp - 2) >> 2;
+        const int m = (warp & 3) * 32 + lane, rp = ew >> 2;
         const uint32_t lanes = tbase + ((uint32_t)((warp & 3) * 32) << 16);
         float bias[NOUT];
 #pragma unroll
@@ -584,7 +591,7 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
     if (!ok && tid == 0) atomicExch(P.err, 1);
     tc::fence_before_sync();
     __syncthreads();
-    if (warp == 1) tc::tmem_dealloc(tbase, kCols);
+    if (warp == kPipeLoadWarps) tc::tmem_dealloc(tbase, kCols);
 }
 
 // per_sm: CTAs per SM the plan's shared memory allows (1 or 2)
