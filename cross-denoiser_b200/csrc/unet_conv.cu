@@ -99,87 +99,88 @@ __host__ __device__ constexpr int conv_cols()
     return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : n <= 256 ? 256 : 512;
 }
 
-// Epilogue of one output row for the pixel x of this thread: bias, ReLU,
-// the ReLU derivative of the layer below (dgrad), bf16 stores, and the fused
-// 2x2 max pooling over rows (r - 1, r) of a tile whose first row is even
-// (prev carries row r - 1; odd = x & 1, the pooled pair is this lane and
+// maxima of two bf16 pairs, a NaN giving the other operand (as fmaxf)
+CD_DEV uint32_t bf2_max(uint32_t a, uint32_t b)
+{
+    uint32_t d;
+    asm("max.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+    return d;
+}
+
+// Epilogue of one output row for the pixel x of this thread: bias, rounding
+// to bf16, ReLU, the ReLU derivative of the layer below (dgrad), stores, and
+// the fused 2x2 max pooling over rows (r - 1, r) of a tile whose first row is
+// even (prev carries row r - 1; odd = x & 1, the pooled pair is this lane and
 // lane ^ 1).  Every lane of the warp calls it (the pooling shuffles).
 // bias: the caller's registers, or null to read P.bias here (kernels with
 // wide rows keep registers for the accumulators).
+// Only the chunks that are stored are worked on, and everything after the
+// bias is done on bf16 pairs (the maxima and the masking give what they give
+// before rounding): on fp32 lanes, all NOUT of them, with a conversion per
+// pooled value the issue slots were 61% busy in the layers of one output
+// chunk (8 -> 8 with pooling at 1920x1080: 38 us, now 30).
 template <int NOUT>
-__device__ __forceinline__ void conv_out_row(const ConvParams &P, float (&v)[NOUT], const float *bias,
-                                             float (&prev)[NOUT], int b, int x, int y, int r, int odd)
+__device__ __forceinline__ void conv_out_row(const ConvParams &P, const float *v, const float *bias,
+                                             uint32_t (&prev)[NOUT / 2], int b, int x, int y, int r, int odd)
 {
     const bool inside = x < P.W && y < P.H;
     const int yi = inside ? y : 0, xi = inside ? x : 0;
-    if (bias) {
+    const int py = y / 2, px = x / 2, PH = P.H / 2, PW = P.W / 2;
+    const bool pooled = (r & 1) && !odd && py < PH && px < PW;
 #pragma unroll
-        for (int j = 0; j < NOUT; ++j) v[j] += bias[j];
-    } else if (P.bias) {
+    for (int c = 0; c < NOUT / 8; ++c) {
+        if (c >= P.d0 + P.d1) break;
+        const bool one = c < P.d0;
+        const size_t at = one ? act_idx(b, yi, c, xi, P.H, P.W, P.d0) : act_idx(b, yi, c - P.d0, xi, P.H, P.W, P.d1);
+        uint4 raw;
+        uint32_t o[4];
 #pragma unroll
-        for (int j = 0; j < NOUT; ++j) v[j] += __ldg(P.bias + j);
-    }
-    if (P.relu) {
-#pragma unroll
-        for (int j = 0; j < NOUT; ++j) v[j] = fmaxf(v[j], 0.f);
-    }
-    if (inside) {
-        // dgrad: multiply by the ReLU derivative of the layer below
-        // (mask0 / mask1 laid out like dst0 / dst1; null = no ReLU)
-#pragma unroll
-        for (int c = 0; c < NOUT / 8; ++c) {
-            if (c >= P.d0 + P.d1) break;
-            const __nv_bfloat16 *m =
-                c < P.d0 ? (P.mask0 ? P.mask0 + act_idx(b, yi, c, xi, P.H, P.W, P.d0) * 8 : nullptr)
-                         : (P.mask1 ? P.mask1 + act_idx(b, yi, c - P.d0, xi, P.H, P.W, P.d1) * 8 : nullptr);
-            if (!m) continue;
-            const uint4 raw = *reinterpret_cast<const uint4 *>(m);
-            const __nv_bfloat16 *mb = reinterpret_cast<const __nv_bfloat16 *>(&raw);
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-                if (!(__bfloat162float(mb[e]) > 0.f)) v[8 * c + e] = 0.f;
-        }
-    }
-    if (inside) {
-#pragma unroll
-        for (int c = 0; c < NOUT / 8; ++c) {
-            if (c >= P.d0 + P.d1) break;
-            uint4 o;
-            __nv_bfloat162 *ob = reinterpret_cast<__nv_bfloat162 *>(&o);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) ob[e] = __floats2bfloat162_rn(v[8 * c + 2 * e], v[8 * c + 2 * e + 1]);
-            __nv_bfloat16 *d = c < P.d0 ? P.dst0 + act_idx(b, yi, c, xi, P.H, P.W, P.d0) * 8
-                                        : P.dst1 + act_idx(b, yi, c - P.d0, xi, P.H, P.W, P.d1) * 8;
-            *reinterpret_cast<uint4 *>(d) = o;
-        }
-    }
-    if (P.pool) {
-        // fused 2x2 max pooling (rows y0 + r - 1, y0 + r; lanes x, x ^ 1),
-        // on the bf16-rounded outputs, as the stored activations are
-        if (r & 1) {
-#pragma unroll
-            for (int j = 0; j < NOUT; ++j) {
-                float m = fmaxf(__bfloat162float(__float2bfloat16_rn(prev[j])),
-                                __bfloat162float(__float2bfloat16_rn(v[j])));
-                m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-                prev[j] = m;
+        for (int e = 0; e < 4; ++e) {
+            const int j = 8 * c + 2 * e;
+            float lo = v[j], hi = v[j + 1];
+            if (bias) {
+                lo += bias[j];
+                hi += bias[j + 1];
+            } else if (P.bias) {
+                lo += __ldg(P.bias + j);
+                hi += __ldg(P.bias + j + 1);
             }
-            const int py = y / 2, px = x / 2, PH = P.H / 2, PW = P.W / 2;
-            if (!odd && py < PH && px < PW) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+            o[e] = *reinterpret_cast<const uint32_t *>(&h);
+        }
+        if (P.relu) {
 #pragma unroll
-                for (int c = 0; c < NOUT / 8; ++c) {
-                    if (c >= P.d0) break;
-                    uint4 o;
-                    __nv_bfloat162 *ob = reinterpret_cast<__nv_bfloat162 *>(&o);
+            for (int e = 0; e < 4; ++e) o[e] = bf2_max(o[e], 0u);
+        }
+        // dgrad: the ReLU derivative of the layer below (mask0 / mask1 laid
+        // out like dst0 / dst1; null = no ReLU)
+        const __nv_bfloat16 *m = one ? P.mask0 : P.mask1;
+        if (m && inside) {
+            raw = *reinterpret_cast<const uint4 *>(m + at * 8);
+            const __nv_bfloat162 *mb = reinterpret_cast<const __nv_bfloat162 *>(&raw);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        ob[e] = __floats2bfloat162_rn(prev[8 * c + 2 * e], prev[8 * c + 2 * e + 1]);
-                    *reinterpret_cast<uint4 *>(P.pool + act_idx(b, py, c, px, PH, PW, P.d0) * 8) = o;
+            for (int e = 0; e < 4; ++e) o[e] &= __hgt2_mask(mb[e], __nv_bfloat162{0, 0});
+        }
+        if (inside)
+            *reinterpret_cast<uint4 *>((one ? P.dst0 : P.dst1) + at * 8) = make_uint4(o[0], o[1], o[2], o[3]);
+        if (P.pool) {
+            // fused 2x2 max pooling (rows y0 + r - 1, y0 + r; lanes x, x ^ 1)
+            // of the rounded outputs
+            if (r & 1) {
+                if (one) {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        o[e] = bf2_max(prev[4 * c + e], o[e]);
+                        o[e] = bf2_max(o[e], __shfl_xor_sync(0xffffffffu, o[e], 1));
+                    }
+                    if (pooled)
+                        *reinterpret_cast<uint4 *>(P.pool + act_idx(b, py, c, px, PH, PW, P.d0) * 8) =
+                            make_uint4(o[0], o[1], o[2], o[3]);
                 }
-            }
-        } else {
+            } else {
 #pragma unroll
-            for (int j = 0; j < NOUT; ++j) prev[j] = v[j];
+                for (int e = 0; e < 4; ++e) prev[4 * c + e] = o[e];
+            }
         }
     }
 }
@@ -318,7 +319,7 @@ __global__ void __launch_bounds__(128) conv3x3_kernel(const ConvParams P)
     } else {
         const int x = x0 + tid;
         const uint32_t lane_base = tbase + ((uint32_t)(warp * 32) << 16);
-        float prev[NOUT];
+        uint32_t prev[NOUT / 2];
         for (int r = 0; r < R; ++r) {
             float v[NOUT];
 #pragma unroll
@@ -365,8 +366,8 @@ cudaError_t launch_rows(const ConvParams &P, int B, cudaStream_t st)
 // i % S (bulk copies; the packed weights once per CTA), one lane of the next
 // warp issues the tile's MMAs into TMEM accumulator buffer i % 2 and commits
 // them to the slot's "empty" and the buffer's "full" barriers, and the other
-// warps (TMEM lanes = pixels) run the epilogue of the buffer, zero it and hand
-// it back through its "empty" barrier.  The epilogue is the longest of the
+// warps (TMEM lanes = pixels) run the epilogue of the buffer: read it, zero it, hand
+// it back through its "empty" barrier, then work on what was read.  The epilogue is the longest of the
 // three per tile, so it has two warps per TMEM lane quadrant, one per pair
 // of output rows (the fused pooling pairs rows 2k, 2k + 1), and two CTAs
 // share an SM where their rings fit half of its shared memory.  A warp issues
@@ -445,13 +446,14 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
     tc::fence_after_sync();
     const uint32_t tbase = *tslot;
     chain_next();
-    // both accumulator buffers start at zero (every MMA accumulates)
+    // the output rows' groups of both accumulator buffers start at zero
+    // (every MMA accumulates; groups 0, 1, R + 2 and R + 3 are never read)
     const int ew = warp - kPipeLoadWarps - 1;   // epilogue warp
     if (ew >= 0) {
         const uint32_t lanes = tbase + ((uint32_t)((warp & 3) * 32) << 16);
         const int rp = ew >> 2;
         for (int k = 0; k < 2; ++k)
-            for (int col = rp * (kGrp / 2); col < (rp + 1) * (kGrp / 2); col += 16)
+            for (int col = (2 * rp + 2) * NOUT; col < (2 * rp + 4) * NOUT; col += 16)
                 tc::tmem_st16_zero(lanes + (uint32_t)(k * kGrp + col));
         tc::tmem_wait_st();
     }
@@ -569,22 +571,24 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
             const int tx = tile % ntx, ty = (tile / ntx) % nty, b = tile / (ntx * nty);
             const int x = tx * kPx + m, y0 = ty * R;
             const uint32_t accl = lanes + (uint32_t)(buf * kGrp);
-            float prev[NOUT];
+            // both rows' sums, then zeros in their place, and the buffer is
+            // the MMAs' again before the rows are worked on
+            float v[2][NOUT];
+            const uint32_t mine = accl + (uint32_t)((2 * rp + 2) * NOUT);
 #pragma unroll
-            for (int r = 2 * rp; r < 2 * rp + 2; ++r) {
-                float v[NOUT];
+            for (int k = 0; k < 2; ++k)
 #pragma unroll
-                for (int j = 0; j < NOUT; j += 16) tc::tmem_ld16(accl + (r + 2) * NOUT + j, v + j);
-                conv_out_row<NOUT>(P, v, bias, prev, b, x, y0 + r, r, lane & 1);
-            }
-            // zero this warp's share of the buffer: its lanes, a column
-            // range per row pair
-            for (int col = rp * (kGrp / 2); col < (rp + 1) * (kGrp / 2); col += 16) tc::tmem_st16_zero(accl + col);
+                for (int j = 0; j < NOUT; j += 16) tc::tmem_ld16(mine + (uint32_t)(k * NOUT + j), v[k] + j);
+#pragma unroll
+            for (int col = 0; col < 2 * NOUT; col += 16) tc::tmem_st16_zero(mine + (uint32_t)col);
             tc::tmem_wait_st();
             tc::fence_before_sync();
             __syncwarp();
             if (lane == 0)
                 asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(&tempty[buf])) : "memory");
+            uint32_t prev[NOUT / 2];
+#pragma unroll
+            for (int k = 0; k < 2; ++k) conv_out_row<NOUT>(P, v[k], bias, prev, b, x, y0 + 2 * rp + k, k, lane & 1);
         }
     }
     ok = __syncthreads_and(ok) != 0;
