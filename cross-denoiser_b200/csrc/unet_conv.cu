@@ -359,21 +359,27 @@ cudaError_t launch_rows(const ConvParams &P, int B, cudaStream_t st)
     }
 }
 
-// Persistent, pipelined form of the ky-stacked convolution.  The same MMAs
-// per tile (R output rows x 128 pixels) as conv3x3_kernel<NOUT, R, true>,
-// with the roles split over warps so that staging, tensor-core work and the
-// epilogue of different tiles overlap: two warps stage tile i into ring slot
-// i % S (bulk copies; the packed weights once per CTA), one lane of the next
-// warp issues the tile's MMAs into TMEM accumulator buffer i % 2 and commits
-// them to the slot's "empty" and the buffer's "full" barriers, and the other
-// warps (TMEM lanes = pixels) run the epilogue of the buffer: read it, zero it, hand
-// it back through its "empty" barrier, then work on what was read.  The epilogue is the longest of the
-// three per tile, so it has two warps per TMEM lane quadrant, one per pair
-// of output rows (the fused pooling pairs rows 2k, 2k + 1), and two CTAs
-// share an SM where their rings fit half of its shared memory.  A warp issues
-// a 2 KB bulk copy about every 150 cycles, so two share a tile's copies (and
-// four in the per-tile kernel): the network's prediction at 1920x1080 takes
-// 261 us, with one 266; a third gave nothing.  Every wait is bounded.
+// Persistent, pipelined form of the ky-stacked convolution.  The sums of
+// conv3x3_kernel<NOUT, R, true> (R output rows x 128 pixels per tile, the same
+// K steps into every output in the same order, MMAs run as issued), with the
+// roles split over warps so that staging, tensor-core work and the epilogue of
+// different tiles overlap: two warps stage tile i into ring slot i % S (bulk
+// copies; the packed weights once per CTA), one lane of the next warp issues
+// the tile's MMAs into TMEM accumulator buffer i % kBufs and commits them to
+// the slot's "empty" and the buffer's "full" barriers, and the other warps
+// (TMEM lanes = pixels) run the epilogue of the buffer: read it, zero it, hand
+// it back through its "empty" barrier, then work on what was read.  An MMA
+// covers only the output rows inside the tile, so a buffer is R row groups (not
+// R + 4) and tiles of 8 rows keep two buffers of both CTAs in TMEM.  Two warps
+// per TMEM lane quadrant share the epilogue, each half of the rows (the fused
+// pooling pairs rows 2k, 2k + 1), and two CTAs share an SM where their rings
+// fit half of its shared memory.  A warp issues a 2 KB bulk copy about every
+// 150 cycles, so two share a tile's copies (and four in the per-tile kernel):
+// the network's prediction at 1920x1080 took 261 us, with one 266; a third
+// gave nothing.  What bounds it: with every other role removed the MMAs alone
+// take 51 of 61 us (24 -> 8 at 2560x1440, 4-row tiles), about 44 cycles each
+// whatever N up to 48 is: the 4 KB A operand read from shared memory.  Every
+// wait is bounded.
 constexpr int kPipeLoadWarps = 2;
 constexpr int kPipeEpiWarps = 8;
 constexpr int kPipeThreads = 32 * (kPipeLoadWarps + 1 + kPipeEpiWarps);
@@ -412,19 +418,21 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
 {
     extern __shared__ __align__(128) uint8_t smem[];
     constexpr int kRowsB = 3 * NOUT;
-    constexpr int kGrp = (R + 4) * NOUT;   // TMEM columns of one accumulator buffer
-    constexpr int kCols = 2 * kGrp <= 32 ? 32 : 2 * kGrp <= 64 ? 64 : 2 * kGrp <= 128 ? 128 : 2 * kGrp <= 256 ? 256 : 512;
-    static_assert(2 * kGrp <= 256, "two CTAs' accumulator buffers fit TMEM");
-    static_assert(R == 2 * (kPipeEpiWarps / 4), "one epilogue warp per lane quadrant and row pair");
+    constexpr int kGrp = R * NOUT;                     // TMEM columns of one accumulator buffer
+    constexpr int kBufs = kGrp <= 64 ? 4 : 2;          // buffers of a CTA
+    constexpr int kCols = 256;                         // two CTAs' buffers fit TMEM
+    static_assert(kBufs * kGrp <= kCols && 2 * kCols <= 512, "two CTAs' accumulator buffers fit TMEM");
+    constexpr int kRowsE = R / (kPipeEpiWarps / 4);    // rows of an epilogue warp
+    constexpr int kUnit = kRowsE % 2 ? 1 : 2;   // rows it holds in registers
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int S = pl.S;
     uint8_t *sB = smem;
     uint8_t *ring = smem + pl.wbytes;
     uint64_t *full = reinterpret_cast<uint64_t *>(ring + (size_t)S * pl.stage);
     uint64_t *empty = full + S;
-    uint64_t *tfull = empty + S;    // [2] accumulator buffer written
-    uint64_t *tempty = tfull + 2;   // [2] accumulator buffer read and zeroed
-    uint64_t *wbar = tempty + 2;
+    uint64_t *tfull = empty + S;        // [kBufs] accumulator buffer written
+    uint64_t *tempty = tfull + kBufs;   // [kBufs] accumulator buffer read (and zeroed)
+    uint64_t *wbar = tempty + kBufs;
     uint32_t *tslot = reinterpret_cast<uint32_t *>(wbar + 1);
 
     chain_wait();
@@ -434,7 +442,7 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
             tc::mbar_init(&full[s], kPipeLoadWarps);
             tc::mbar_init(&empty[s], 1);
         }
-        for (int k = 0; k < 2; ++k) {
+        for (int k = 0; k < kBufs; ++k) {
             tc::mbar_init(&tfull[k], 1);
             tc::mbar_init(&tempty[k], kPipeEpiWarps);
         }
@@ -446,14 +454,13 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
     tc::fence_after_sync();
     const uint32_t tbase = *tslot;
     chain_next();
-    // the output rows' groups of both accumulator buffers start at zero
-    // (every MMA accumulates; groups 0, 1, R + 2 and R + 3 are never read)
+    // the buffers start at zero (every MMA accumulates)
     const int ew = warp - kPipeLoadWarps - 1;   // epilogue warp
     if (ew >= 0) {
         const uint32_t lanes = tbase + ((uint32_t)((warp & 3) * 32) << 16);
         const int rp = ew >> 2;
-        for (int k = 0; k < 2; ++k)
-            for (int col = (2 * rp + 2) * NOUT; col < (2 * rp + 4) * NOUT; col += 16)
+        for (int k = 0; k < kBufs; ++k)
+            for (int col = rp * kRowsE * NOUT; col < (rp + 1) * kRowsE * NOUT; col += 16)
                 tc::tmem_st16_zero(lanes + (uint32_t)(k * kGrp + col));
         tc::tmem_wait_st();
     }
@@ -512,7 +519,6 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
     } else if (warp == kPipeLoadWarps) {
         // ---- MMA issue (one thread) ----
         if (lane == 0) {
-            const uint32_t idesc = tc::idesc_bf16(kPx, kRowsB);
             // per K step: A descriptor of row 0 relative to a slot (start
             // field = byte offset / 16), its row stride in 16-byte units,
             // and the B descriptor
@@ -528,9 +534,9 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
             }
             ok = tc::mbar_wait(wbar, 0, kWaitIter);
             for (int i = 0; ok && i < ntile; ++i) {
-                const int s = i % S, buf = i & 1;
+                const int s = i % S, buf = i % kBufs;
                 if (!tc::mbar_wait(&full[s], (uint32_t)(i / S) & 1u, kWaitIter) ||
-                    (i >= 2 && !tc::mbar_wait(&tempty[buf], (uint32_t)(i / 2 - 1) & 1u, kWaitIter))) {
+                    (i >= kBufs && !tc::mbar_wait(&tempty[buf], (uint32_t)(i / kBufs - 1) & 1u, kWaitIter))) {
                     ok = false;
                     break;
                 }
@@ -542,27 +548,34 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
                 uint64_t at[NST];
 #pragma unroll
                 for (int k = 0; k < NST; ++k) at[k] = ad[k] + sbase;
+                // input row r is tap ky = 2, 1, 0 (blocks 0, 1, 2 of B) of
+                // output rows r - 2, r - 1, r: those inside the tile
 #pragma unroll
-                for (int r = 0; r < R + 2; ++r)
+                for (int r = 0; r < R + 2; ++r) {
+                    const int j0 = r < 2 ? 2 - r : 0, j1 = r > R - 1 ? R + 1 - r : 2;
+                    const uint32_t idesc = tc::idesc_bf16(kPx, (j1 - j0 + 1) * NOUT);
 #pragma unroll
                     for (int k = 0; k < NST; ++k)
-                        tc::mma_bf16(acc + r * NOUT, at[k] + (uint64_t)(r * rs[k]), bd[k], idesc, 1u);
+                        tc::mma_bf16(acc + (r + j0 - 2) * NOUT, at[k] + (uint64_t)(r * rs[k]),
+                                     bd[k] + (uint64_t)(j0 * NOUT), idesc, 1u);
+                }
                 tc::commit(&empty[s]);
                 tc::commit(&tfull[buf]);
             }
         }
         ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
     } else {
-        // ---- epilogue: TMEM lane m = pixel x0 + m, output rows 2 rp, 2 rp + 1 ----
+        // ---- epilogue: TMEM lane m = pixel x0 + m, kRowsE output rows from
+        // rp * kRowsE ----
         const int m = (warp & 3) * 32 + lane, rp = ew >> 2;
         const uint32_t lanes = tbase + ((uint32_t)((warp & 3) * 32) << 16);
         float bias[NOUT];
 #pragma unroll
         for (int j = 0; j < NOUT; ++j) bias[j] = P.bias ? __ldg(P.bias + j) : 0.f;   // zeros: no bias
         for (int i = 0; i < ntile; ++i) {
-            const int buf = i & 1, tile = first + i * stride;
+            const int buf = i % kBufs, tile = first + i * stride;
             bool got = true;
-            if (lane == 0) got = tc::mbar_wait(&tfull[buf], (uint32_t)(i / 2) & 1u, kWaitIter);
+            if (lane == 0) got = tc::mbar_wait(&tfull[buf], (uint32_t)(i / kBufs) & 1u, kWaitIter);
             if (!__shfl_sync(0xffffffffu, got ? 1 : 0, 0)) {
                 ok = false;
                 break;
@@ -570,25 +583,34 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
             tc::fence_after_sync();
             const int tx = tile % ntx, ty = (tile / ntx) % nty, b = tile / (ntx * nty);
             const int x = tx * kPx + m, y0 = ty * R;
-            const uint32_t accl = lanes + (uint32_t)(buf * kGrp);
-            // both rows' sums, then zeros in their place, and the buffer is
-            // the MMAs' again before the rows are worked on
-            float v[2][NOUT];
-            const uint32_t mine = accl + (uint32_t)((2 * rp + 2) * NOUT);
-#pragma unroll
-            for (int k = 0; k < 2; ++k)
-#pragma unroll
-                for (int j = 0; j < NOUT; j += 16) tc::tmem_ld16(mine + (uint32_t)(k * NOUT + j), v[k] + j);
-#pragma unroll
-            for (int col = 0; col < 2 * NOUT; col += 16) tc::tmem_st16_zero(mine + (uint32_t)col);
-            tc::tmem_wait_st();
-            tc::fence_before_sync();
-            __syncwarp();
-            if (lane == 0)
-                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(&tempty[buf])) : "memory");
+            const uint32_t mine = lanes + (uint32_t)(buf * kGrp + rp * kRowsE * NOUT);
             uint32_t prev[NOUT / 2];
 #pragma unroll
-            for (int k = 0; k < 2; ++k) conv_out_row<NOUT>(P, v[k], bias, prev, b, x, y0 + 2 * rp + k, k, lane & 1);
+            for (int u = 0; u < kRowsE; u += kUnit) {
+                float v[kUnit][NOUT];
+#pragma unroll
+                for (int k = 0; k < kUnit; ++k)
+#pragma unroll
+                    for (int j = 0; j < NOUT; j += 16)
+                        tc::tmem_ld16(mine + (uint32_t)((u + k) * NOUT + j), v[k] + j);
+                if (u + kUnit == kRowsE) {
+                    // all read: zeros in place of the sums, and the buffer is
+                    // the MMAs' again before the last rows are worked on
+#pragma unroll
+                    for (int col = 0; col < kRowsE * NOUT; col += 16) tc::tmem_st16_zero(mine + (uint32_t)col);
+                    tc::tmem_wait_st();
+                    tc::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0)
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(tc::smem_u32(&tempty[buf]))
+                                     : "memory");
+                }
+#pragma unroll
+                for (int k = 0; k < kUnit; ++k) {
+                    const int r = rp * kRowsE + u + k;
+                    conv_out_row<NOUT>(P, v[k], bias, prev, b, x, y0 + r, r, lane & 1);
+                }
+            }
         }
     }
     ok = __syncthreads_and(ok) != 0;
@@ -598,6 +620,14 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
     if (warp == kPipeLoadWarps) tc::tmem_dealloc(tbase, kCols);
 }
 
+inline int sm_count()
+{
+    int dev = 0, nsm = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    return nsm;
+}
+inline int conv_tiles(const ConvParams &P, int B, int R) { return B * ((P.W + kPx - 1) / kPx) * ((P.H + R - 1) / R); }
+
 // per_sm: CTAs per SM the plan's shared memory allows (1 or 2)
 template <int NOUT, int R, int NST>
 cudaError_t launch_pipe_t(const ConvParams &P, const ConvPipePlan &pl, int per_sm, int B, cudaStream_t st)
@@ -606,9 +636,7 @@ cudaError_t launch_pipe_t(const ConvParams &P, const ConvPipePlan &pl, int per_s
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem);
     if (e != cudaSuccess) return e;
     const int ntx = (P.W + kPx - 1) / kPx, nty = (P.H + R - 1) / R, ntiles = B * ntx * nty;
-    int dev = 0, nsm = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    const int grid = ntiles < per_sm * nsm ? ntiles : per_sm * nsm;
+    const int nsm = sm_count(), grid = ntiles < per_sm * nsm ? ntiles : per_sm * nsm;
     return launch_chained(conv3x3_pipe_kernel<NOUT, R, NST>, grid, kPipeThreads, pl.smem, st, P, pl, ntx, nty,
                           ntiles);
 }
@@ -1208,6 +1236,26 @@ cudaError_t launch_conv3x3(const ConvParams &P, int B, int nout, cudaStream_t st
     if (P.stacked) {
         constexpr int Rs = kConvRowsStacked;
         if (nout == 16 && tma::persistent_enabled() && pipe_steps_supported(P.nsteps)) {
+            // Tall tiles, 8 rows for one or two input chunks, 6 for three
+            // (what two CTAs' rings of two slots leave room for; 6 rows give
+            // an epilogue warp three, so no pooling), once every CTA has two
+            // of them.  An MMA costs the same for one to three output rows,
+            // so a tile's cost is its R + 2 input rows: per output row 1.25
+            // and 1.33 of them against 1.5.  15 -> 8 at 1280x720 17.2 -> 16.2
+            // us, at 3840x2160 97 -> 77; 24 -> 8 at 3840x2160 127 -> 111; at
+            // 1024x720 (fewer tiles than that) no gain.  Forward only (a
+            // bias): in the backward pass, beside the weight gradients, the
+            // U-Net step at 2560x1440 took 1350 us with them, 1329 without.
+            const int two_each = 2 * 2 * sm_count(), nch = P.c0 + P.c1;
+            if (P.bias && nch <= 2 && conv_tiles(P, B, 8) >= two_each) {
+                const ConvPipePlan p8 = conv_pipe_plan(P.nsteps, 3 * 16, P.c0, P.c1, 8, kPipeSmem2);
+                if (p8.S >= 2 && P.nsteps == 2) return launch_pipe_t<16, 8, 2>(P, p8, 2, B, st);
+                if (p8.S >= 2 && P.nsteps == 3) return launch_pipe_t<16, 8, 3>(P, p8, 2, B, st);
+            }
+            if (P.bias && !P.pool && P.nsteps == 5 && conv_tiles(P, B, 6) >= two_each) {
+                const ConvPipePlan p6 = conv_pipe_plan(P.nsteps, 3 * 16, P.c0, P.c1, 6, kPipeSmem2);
+                if (p6.S >= 2) return launch_pipe_t<16, 6, 5>(P, p6, 2, B, st);
+            }
             const ConvPipePlan p2 = conv_pipe_plan(P.nsteps, 3 * 16, P.c0, P.c1, Rs, kPipeSmem2);
             if (p2.S >= 2) return launch_pipe<16, Rs>(P, p2, 2, B, st);
             const ConvPipePlan p1 = conv_pipe_plan(P.nsteps, 3 * 16, P.c0, P.c1, Rs, kPipeSmem);
