@@ -52,6 +52,16 @@ CD_DEV bool depth_normal_ok(float Z, float Zp, float fwZ, float3 n, float3 np, f
     if (depth_bad) return false;
     const float dx = __fsub_rn(n.x, np.x), dy = __fsub_rn(n.y, np.y), dz = __fsub_rn(n.z, np.z);
     const float dd = __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
+    // Away from the threshold the squares decide: t is 16 S^2 to a few parts
+    // in 2^24, dist the root of dd to one, so a margin of 1e-4 either way
+    // settles what the root and the doubles below would say.  (With S out of
+    // range, NaN or close to the threshold neither line returns.)
+    const float s32 = __fadd_rn(fwN, 1e-2f);
+    if (s32 >= 0x1p-10f && s32 <= 0x1p20f) {
+        const float t = __fmul_rn(16.f, __fmul_rn(s32, s32));
+        if (dd <= __fmul_rn(t, 0.9999f)) return true;
+        if (dd >= __fmul_rn(t, 1.0001f)) return false;
+    }
     const float dist = __fsqrt_rn(dd);
     const double S = __dadd_rn((double)fwN, 1e-2);
     const bool normal_bad = (S >= 0x1p-900 && S <= 0x1p900 && dist <= 0x1p100f)
@@ -226,7 +236,52 @@ CD_DEV float bilinear(float ppx, float ppy, unsigned vmask, float w[4])
     return sumw;
 }
 
-__global__ void __launch_bounds__(256) reproject_decide_kernel(
+// The 3x3 box around (ipx, ipy): bit k set where tap k is inside the image
+// and its previous opacity is not zero (read without the batch offset, as the
+// reference does: ops/reproject.cu.cc:191).  All loads are issued before the
+// first is used: tap by tap, each behind the one before, they were a chain of
+// 18 memory latencies for any warp with one such pixel.  With that and the
+// squared normal test the decision kernel takes 47 us at 1920x1080, 52
+// before; 48 registers (five blocks, its former occupancy), at the 56 it
+// would take 50.5.  The gather kernel keeps the chain: its sums need the
+// values too, and at five blocks with this form it took 63 us against 59.
+CD_DEV unsigned box_opacity(const float *__restrict__ popac, int ipx, int ipy, int W, int H)
+{
+    float po[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const int qx = ipx + (k % 3) - 1, qy = ipy + (k / 3) - 1;
+        po[k] = qx >= W || qx < 0 || qy >= H || qy < 0 ? 0.f : __ldg(popac + (size_t)qy * W + qx);
+    }
+    unsigned m = 0u;
+#pragma unroll
+    for (int k = 0; k < 9; ++k)
+        if (po[k] != 0.f) m |= 1u << k;
+    return m;
+}
+
+// Of row j of that box, the taps among `open` (three bits) that pass the
+// depth and normal test.
+CD_DEV unsigned box_row(unsigned open, int j, const float *__restrict__ plinz, const float *__restrict__ pnrm,
+                        size_t base, int ipx, int ipy, int W, float Z, float fwZ, float3 n, float fwN)
+{
+    float zp[3];
+    float3 np[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        if (open & (1u << i)) {
+            const size_t q = base + (size_t)(ipy + j - 1) * W + (ipx + i - 1);
+            zp[i] = __ldg(plinz + 3 * q);
+            np[i] = ld3(pnrm, q);
+        }
+    unsigned ok = 0u;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        if ((open & (1u << i)) && depth_normal_ok(Z, zp[i], fwZ, n, np[i], fwN)) ok |= 1u << i;
+    return ok;
+}
+
+__global__ void __launch_bounds__(256, 5) reproject_decide_kernel(
     const float *__restrict__ mvec, const float *__restrict__ linz, const float *__restrict__ plinz,
     const float *__restrict__ nrm, const float *__restrict__ pnrm, const float *__restrict__ pnfw,
     const float *__restrict__ opac, const float *__restrict__ popac, uint8_t *__restrict__ success, int H, int W)
@@ -271,16 +326,10 @@ __global__ void __launch_bounds__(256) reproject_decide_kernel(
         if (vmask && bilinear(ppx, ppy, vmask, w) >= 0.01f) {
             code = (uint8_t)(kModeBilinear | vmask);
         } else if (border_ok) {
-#pragma unroll
-            for (int k = 0; k < 9 && code == 0; ++k) {
-                const int qx = ipx + (k % 3) - 1, qy = ipy + (k / 3) - 1;
-                if (qx >= W || qx < 0 || qy >= H || qy < 0) continue;
-                // the reference reads prev_opacity here without the batch
-                // offset (ops/reproject.cu.cc:191)
-                if (__ldg(popac + (size_t)qy * W + qx) == 0.f) continue;
-                const size_t q = base + (size_t)qy * W + qx;
-                if (depth_normal_ok(Z, __ldg(plinz + 3 * q), fwZ, n, ld3(pnrm, q), fwN)) code = kModeBox;
-            }
+            const unsigned open = box_opacity(popac, ipx, ipy, W, H);
+#pragma unroll 1
+            for (int j = 0; j < 3 && code == 0; ++j)
+                if (box_row((open >> (3 * j)) & 7u, j, plinz, pnrm, base, ipx, ipy, W, Z, fwZ, n, fwN)) code = kModeBox;
         }
     }
     success[c] = code;
