@@ -71,7 +71,7 @@ KERNELS_PER_CALL = {
     "cd_reproject": 1,   # 2 for the three 3-channel tensors of the step (ops.reproject passes the count)
     "cd_erode3x3": 1, "cd_temporal_screening": 1, "cd_erode_temporal_screening": 1,
     "cd_prepare_input": 1, "cd_aggregation_loss": 2, "cd_filter_aggregate": 2,
-    "cd_unet_forward": 22, "cd_unet_backward": 25, "cd_adam_update": 2, "cd_unet_conv3x3": 2,
+    "cd_unet_forward": 14, "cd_unet_backward": 24, "cd_adam_update": 2, "cd_unet_conv3x3": 2,
     "cd_unet_conv3x3_wgrad": 2,
 }
 LAUNCHES = {"count": 0}
