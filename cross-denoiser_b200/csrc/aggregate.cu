@@ -107,7 +107,7 @@ CD_DEV void block_partial(float v, float *partial, int nthreads)
     block_partial_at(v, partial, (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x, nthreads);
 }
 
-__global__ void __launch_bounds__(1024) loss_reduce_kernel(const float *__restrict__ partial, int n,
+__global__ void __launch_bounds__(1024) loss_reduce_kernel(const float *partial, int n,
                                                            float inv_n, float *__restrict__ avg)
 {
     chain_wait();
@@ -125,15 +125,15 @@ __global__ void __launch_bounds__(1024) loss_reduce_kernel(const float *__restri
     }
 }
 
-__global__ void __launch_bounds__(256) log1p_kernel(const float *__restrict__ a, const float *__restrict__ b,
+__global__ void __launch_bounds__(256) log1p_kernel(const float *a, const float *b,
                                                     float *__restrict__ ya, float *__restrict__ yb, size_t n)
 {
     chain_wait();
     chain_next();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) {
-        ya[i] = log1pf(__ldg(a + i));
-        yb[i] = log1pf(__ldg(b + i));
+        ya[i] = log1pf(a[i]);
+        yb[i] = log1pf(b[i]);
     }
 }
 
@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(256) log1p_kernel(const float *__restrict__ a,
 // all loads issued before the first log1pf, so that enough bytes are in
 // flight to cover the DRAM latency.
 constexpr int kLogVec = 2;
-__global__ void __launch_bounds__(256) log1p4_kernel(const float4 *__restrict__ a, const float4 *__restrict__ b,
+__global__ void __launch_bounds__(256) log1p4_kernel(const float4 *a, const float4 *b,
                                                      float4 *__restrict__ ya, float4 *__restrict__ yb, size_t n4)
 {
     chain_wait();
@@ -152,8 +152,8 @@ __global__ void __launch_bounds__(256) log1p4_kernel(const float4 *__restrict__ 
     for (int k = 0; k < kLogVec; ++k) {
         const size_t i = i0 + (size_t)k * blockDim.x;
         if (i < n4) {
-            va[k] = __ldg(a + i);
-            vb[k] = __ldg(b + i);
+            va[k] = a[i];
+            vb[k] = b[i];
         }
     }
 #pragma unroll
@@ -186,20 +186,20 @@ __global__ void __launch_bounds__(256) aggregation_kernel(AggPtrs P, int H, int 
         AggIn in;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
-            in.s1[k] = __ldg(P.s1 + 3 * p + k);
-            in.s2[k] = __ldg(P.s2 + 3 * p + k);
-            in.prev[k] = __ldg(P.prev + 3 * p + k);
-            in.l1[k] = __ldg(P.l1 + 3 * p + k);
-            in.l2[k] = __ldg(P.l2 + 3 * p + k);
-            in.pl1[k] = __ldg(P.pl1 + 3 * p + k);
-            in.pl2[k] = __ldg(P.pl2 + 3 * p + k);
+            in.s1[k] = P.s1[3 * p + k];
+            in.s2[k] = P.s2[3 * p + k];
+            in.prev[k] = P.prev[3 * p + k];
+            in.l1[k] = P.l1[3 * p + k];
+            in.l2[k] = P.l2[3 * p + k];
+            in.pl1[k] = P.pl1[3 * p + k];
+            in.pl2[k] = P.pl2[3 * p + k];
         }
-        in.w1 = __ldg(P.w1 + p);
-        in.w2 = __ldg(P.w2 + p);
-        in.alpha = __ldg(P.alpha + p);
-        in.succ = __ldg(P.succ + p);
-        in.succ_prev = __ldg(P.succ_prev + p);
-        in.opac = __ldg(P.opac + p);
+        in.w1 = P.w1[p];
+        in.w2 = P.w2[p];
+        in.alpha = P.alpha[p];
+        in.succ = P.succ[p];
+        in.succ_prev = P.succ_prev[p];
+        in.opac = P.opac[p];
         const AggOut r = aggregate(in, inv_n);
         st3(P.out_log, p, make_float3(r.out_log[0], r.out_log[1], r.out_log[2]));
         st3(P.out, p, make_float3(r.out[0], r.out[1], r.out[2]));
@@ -238,14 +238,14 @@ CD_DEV float filter_epilogue(const fsw::Sums &s, const fsw::Centre &c, const Agg
     in.l2[2] = fsw::lo(c.ab_z);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        in.prev[k] = __ldg(P.prev + 3 * p + k);
-        in.pl1[k] = __ldg(P.pl1 + 3 * p + k);      // prev_label1 = prev_ols2
-        in.pl2[k] = __ldg(P.pl2 + 3 * p + k);      // prev_label2 = prev_ols1
+        in.prev[k] = P.prev[3 * p + k];
+        in.pl1[k] = P.pl1[3 * p + k];      // prev_label1 = prev_ols2
+        in.pl2[k] = P.pl2[3 * p + k];      // prev_label2 = prev_ols1
     }
-    in.alpha = __ldg(P.alpha + p);
-    in.succ = __ldg(P.succ + p);
-    in.succ_prev = __ldg(P.succ_prev + p);
-    in.opac = __ldg(P.opac + p);
+    in.alpha = P.alpha[p];
+    in.succ = P.succ[p];
+    in.succ_prev = P.succ_prev[p];
+    in.opac = P.opac[p];
     const AggOut r = aggregate(in, inv_n);
     st3(P.out_log, p, make_float3(r.out_log[0], r.out_log[1], r.out_log[2]));
     st3(P.out, p, make_float3(r.out[0], r.out[1], r.out[2]));
@@ -270,8 +270,8 @@ CD_DEV float filter_epilogue(const fsw::Sums &s, const fsw::Centre &c, const Agg
 // ---------------------------------------------------------------------------
 template <int HW>
 __global__ void __launch_bounds__(256, 2) filter_aggregate_kernel(
-    const float *__restrict__ imga, const float *__restrict__ imgb, const float *__restrict__ albedo,
-    const float *__restrict__ normal, const float *__restrict__ band, AggPtrs P,
+    const float *imga, const float *imgb, const float *albedo,
+    const float *normal, const float *band, AggPtrs P,
     float *__restrict__ gband, int H, int W, int hw_rt, float inv_n)
 {
     chain_wait();

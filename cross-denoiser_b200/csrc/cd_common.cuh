@@ -17,7 +17,11 @@ CD_DEV int mirror(int i, int n) { return (i >= n) ? 2 * n - 2 - i : abs(i); }
 // for negative a it is one above the mathematical ceiling when a % b != 0.
 CD_DEV int idivup(int a, int b) { return (a % b != 0) ? (a / b + 1) : (a / b); }
 
-CD_DEV float3 ld3(const float *p, size_t i)
+// ld3: a plain load, for any kernel (launch.cuh: a chained kernel has no
+// other).  ldg3: the non-coherent path, only where the kernel is launched
+// after the end of everything that writes the buffer.
+CD_DEV float3 ld3(const float *p, size_t i) { return make_float3(p[3 * i], p[3 * i + 1], p[3 * i + 2]); }
+CD_DEV float3 ldg3(const float *p, size_t i)
 {
     return make_float3(__ldg(p + 3 * i), __ldg(p + 3 * i + 1), __ldg(p + 3 * i + 2));
 }

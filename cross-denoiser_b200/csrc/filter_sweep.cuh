@@ -182,8 +182,8 @@ CD_DEV Centre centre(const ulonglong2 *tile, int hw, const float *band5)
     c.an_x = r[1].y;
     c.an_y = r[2].x;
     c.an_z = r[2].y;
-    const float b0 = __ldg(band5), b1 = __ldg(band5 + 1), b2 = __ldg(band5 + 2);
-    const float b3 = __ldg(band5 + 3), b4 = __ldg(band5 + 4);
+    const float b0 = band5[0], b1 = band5[1], b2 = band5[2];
+    const float b3 = band5[3], b4 = band5[4];
     c.nb01 = pack(-b0, -b1);
     c.nb2 = pack(-b2, -b2);
     c.nb3 = pack(-b3, -b3);

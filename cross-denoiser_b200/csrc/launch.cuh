@@ -6,6 +6,13 @@
 //   * chain_wait() comes before its first access to global memory, read or
 //     write: it returns once the kernel before it has completed and its
 //     writes are visible (that kernel's own chain_wait orders the ones before);
+//   * its inputs are read with plain loads through pointers without
+//     __restrict__ (or by cp.async, bulk and TMA copies): it is resident while
+//     its predecessor writes them, so they are not read-only for its lifetime,
+//     as __ldg and the loads that the compiler may make of const __restrict__
+//     pointers require; and such loads, which memory is held never to change
+//     under, are not tied down by chain_wait()'s clobber.  __restrict__ stays
+//     on pointers that a kernel only writes;
 //   * chain_next() lets the next kernel's CTAs start; a kernel that allocates
 //     TMEM does so after chain_wait() and calls chain_next() after the
 //     allocation, so no waiting CTA ever holds TMEM that an earlier kernel's

@@ -40,8 +40,8 @@ constexpr int kBeta = kP * 3;    // floats per centre and buffer
 constexpr int kVX = 32, kVY = 8;
 constexpr int kVRow = 3 * (kVX + 8), kVTH = kVY + 2;   // footprint row: 40 pixels x 3 floats
 
-__global__ void __launch_bounds__(kVX * kVY) variance_kernel(const float *__restrict__ imga,
-                                                             const float *__restrict__ imgb,
+__global__ void __launch_bounds__(kVX * kVY) variance_kernel(const float *imga,
+                                                             const float *imgb,
                                                              float *__restrict__ vara,
                                                              float *__restrict__ varb,
                                                              float *__restrict__ sda,
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(kVX * kVY) variance_kernel(const float *__rest
         const int f = 3 * xa + 4 * lane;   // float offset in the image row
         v[k] = make_float4(0.f, 0.f, 0.f, 0.f);   // outside the image: never read
         if (rr < kRows && 4 * lane < kVRow && gy >= 0 && gy < H && f >= 0 && f + 4 <= 3 * W)
-            v[k] = __ldg(reinterpret_cast<const float4 *>((buf ? imgb : imga) + 3 * (base + (size_t)gy * W) + f));
+            v[k] = *reinterpret_cast<const float4 *>((buf ? imgb : imga) + 3 * (base + (size_t)gy * W) + f);
     }
 #pragma unroll
     for (int k = 0; k < kIt; ++k) {
@@ -110,8 +110,8 @@ __global__ void __launch_bounds__(kVX * kVY) variance_kernel(const float *__rest
     }
 }
 
-__global__ void __launch_bounds__(256) variance_px_kernel(const float *__restrict__ imga,
-                                                       const float *__restrict__ imgb,
+__global__ void __launch_bounds__(256) variance_px_kernel(const float *imga,
+                                                       const float *imgb,
                                                        float *__restrict__ vara,
                                                        float *__restrict__ varb,
                                                        float *__restrict__ sda,
@@ -531,8 +531,8 @@ __global__ void __launch_bounds__(kThreads, 8) regression_kernel(
     // centre values, read directly (clamped for lanes past the last centre)
     const int ci = min(i0 + lane, Ws - 1);
     const size_t c = (size_t)cy * W + (size_t)ci * sp;
-    const float3 fc = ld3(buf ? imgb : imga, c);
-    const float3 alc = ld3(albedo, c), nrc = ld3(normal, c);
+    const float3 fc = ldg3(buf ? imgb : imga, c);
+    const float3 alc = ldg3(albedo, c), nrc = ldg3(normal, c);
     const float vc = __ldg((buf ? varb : vara) + c), sdc = __ldg((buf ? sdb : sda) + c);
     const Centre cen = {x2::pack(fc.x, fc.y), x2::pack(alc.x, alc.y), x2::pack(nrc.x, nrc.y), fc.z, alc.z, nrc.z,
                         vc, sdc};
@@ -644,11 +644,11 @@ struct ReconPixel {
 // them reaches are a uniform branch.
 template <int NP>
 __global__ void __launch_bounds__(kRX * kRThreadRows, NP == 2 ? 4 : 1) recon_kernel(
-    const float *__restrict__ imga, const float *__restrict__ imgb,
-    const float *__restrict__ albedo, const float *__restrict__ normal,
-    const float *__restrict__ vara, const float *__restrict__ varb,
-    const float *__restrict__ sda, const float *__restrict__ sdb,
-    const float *__restrict__ beta, float *__restrict__ outa, float *__restrict__ outb,
+    const float *imga, const float *imgb,
+    const float *albedo, const float *normal,
+    const float *vara, const float *varb,
+    const float *sda, const float *sdb,
+    const float *beta, float *__restrict__ outa, float *__restrict__ outb,
     float *__restrict__ state, int H, int W, int hw, int sp, int rs)
 {
     chain_wait();
@@ -688,15 +688,15 @@ __global__ void __launch_bounds__(kRX * kRThreadRows, NP == 2 ? 4 : 1) recon_ker
         const int n = e / 9, f = e - 9 * n;
         const int iy = cy_lo + n / ncx, ix = cx_lo + n % ncx;
         const size_t cb = ((size_t)iy * Ws + ix) * kBeta + 2 * f;
-        rec[n * kRec + f] = make_float4(__ldg(betaA + cb), __ldg(betaB + cb), __ldg(betaA + cb + 1), __ldg(betaB + cb + 1));
+        rec[n * kRec + f] = make_float4(betaA[cb], betaB[cb], betaA[cb + 1], betaB[cb + 1]);
     }
     for (int n = tid; n < nc; n += kBlock) {
         const int iy = cy_lo + n / ncx, ix = cx_lo + n % ncx;
         const size_t t = (size_t)(iy * sp) * W + ix * sp;
         const float3 fa = ld3(imga, t), fb = ld3(imgb, t), al = ld3(albedo, t), nr = ld3(normal, t);
         rec[n * kRec + 9] = make_float4(fa.x, fb.x, fa.y, fb.y);
-        rec[n * kRec + 10] = make_float4(fa.z, fb.z, __ldg(vara + t), __ldg(varb + t));
-        rec[n * kRec + 11] = make_float4(__ldg(sda + t), __ldg(sdb + t), al.x, al.y);
+        rec[n * kRec + 10] = make_float4(fa.z, fb.z, vara[t], varb[t]);
+        rec[n * kRec + 11] = make_float4(sda[t], sdb[t], al.x, al.y);
         rec[n * kRec + 12] = make_float4(al.z, nr.x, nr.y, nr.z);
     }
     __syncthreads();
@@ -722,8 +722,8 @@ __global__ void __launch_bounds__(kRX * kRThreadRows, NP == 2 ? 4 : 1) recon_ker
         q.f0 = pack(fa.x, fb.x);
         q.f1 = pack(fa.y, fb.y);
         q.f2 = pack(fa.z, fb.z);
-        q.var = pack(__ldg(vara + p), __ldg(varb + p));
-        q.sd = pack(__ldg(sda + p), __ldg(sdb + p));
+        q.var = pack(vara[p], varb[p]);
+        q.sd = pack(sda[p], sdb[p]);
         q.o0 = q.o1 = q.o2 = q.sw = 0ull;   // +0.0f in both lanes
     }
     const f2 k1e2 = pack(1e-2f, 1e-2f), k1e4 = pack(1e-4f, 1e-4f), k1e7 = pack(1e-7f, 1e-7f);

@@ -62,7 +62,7 @@ struct GArgs {
     bool u_rows;   // pass 4 also writes u as [buffer][centre][18] (for the unstaged tap pass)
 };
 
-CD_DEV float3 f3(const float *p, size_t i) { return ld3(p, i); }
+CD_DEV float3 f3(const float *p, size_t i) { return ldg3(p, i); }
 CD_DEV void add3(float *p, size_t i, float3 v)
 {
     p[3 * i] += v.x;
@@ -747,7 +747,7 @@ __global__ void __launch_bounds__(64, 7) recon_grad_centre_rows_kernel(GArgs A)
         beta[k] = __ldg(betap + k);
         gb[k] = 0.f;
     }
-    const float3 fc = ld3(X ? imgb : imga, c), ac = ld3(alb, c), nc = ld3(nrm, c);
+    const float3 fc = ldg3(X ? imgb : imga, c), ac = ldg3(alb, c), nc = ldg3(nrm, c);
     const float vc = __ldg((X ? varb : vara) + c), sc = __ldg((X ? sdb : sda) + c);
     float3 gf = make_float3(0.f, 0.f, 0.f), galb = gf, gnn = gf;
     float gs = 0.f, gv = 0.f;
@@ -909,7 +909,7 @@ __global__ void __launch_bounds__(64, 8) regression_grad_centre_kernel(GArgs A)
             for (int k = 0; k < kBeta; ++k) ug[k] = u[k];
         }
     }
-    const float3 fc = ld3(X ? imgb : imga, c), ac = ld3(alb, c), nc = ld3(nrm, c);
+    const float3 fc = ldg3(X ? imgb : imga, c), ac = ldg3(alb, c), nc = ldg3(nrm, c);
     const float vc = __ldg((X ? varb : vara) + c), sc = __ldg((X ? sdb : sda) + c);
     const int gfi = X ? 1 : 0, gyi = X ? 0 : 1;   // own features + variance, target
 

@@ -72,10 +72,10 @@ CD_DEV bool depth_normal_ok(float Z, float Zp, float fwZ, float3 n, float3 np, f
 
 template <int kN, int kC>
 __global__ void __launch_bounds__(256) reproject_kernel(
-    const float *__restrict__ mvec, ReprojectList list, const float *__restrict__ linz,
-    const float *__restrict__ plinz, const float *__restrict__ nrm,
-    const float *__restrict__ pnrm, const float *__restrict__ pnfw,
-    const float *__restrict__ opac, const float *__restrict__ popac,
+    const float *mvec, ReprojectList list, const float *linz,
+    const float *plinz, const float *nrm,
+    const float *pnrm, const float *pnfw,
+    const float *opac, const float *popac,
     uint8_t *__restrict__ success, int H, int W)
 {
     chain_wait();
@@ -96,9 +96,9 @@ __global__ void __launch_bounds__(256) reproject_kernel(
     int lx = 0, ly = 0, ipx = 0, ipy = 0;
 
     // own-pixel inputs loaded together, not behind the opacity test
-    const float op = __ldg(opac + c), mx = __ldg(mvec + 3 * c), my = __ldg(mvec + 3 * c + 1);
-    const float fwN = __ldg(pnfw + 3 * c + 1);
-    const float Z = __ldg(linz + 3 * c), fwZ = __ldg(linz + 3 * c + 1);
+    const float op = opac[c], mx = mvec[3 * c], my = mvec[3 * c + 1];
+    const float fwN = pnfw[3 * c + 1];
+    const float Z = linz[3 * c], fwZ = linz[3 * c + 1];
     const float3 n = ld3(nrm, c);
     if (op != 0.f) {
         const float fW = (float)W, fH = (float)H, fx = (float)cx, fy = (float)cy;
@@ -123,8 +123,8 @@ __global__ void __launch_bounds__(256) reproject_kernel(
                 po[s] = 0.f;
                 if (qx >= W || qx < 0 || qy >= H || qy < 0) continue;
                 const size_t q = base + (size_t)qy * W + qx;
-                po[s] = __ldg(popac + q);
-                zp[s] = __ldg(plinz + 3 * q);
+                po[s] = popac[q];
+                zp[s] = plinz[3 * q];
                 np[s] = ld3(pnrm, q);
             }
 #pragma unroll
@@ -156,9 +156,9 @@ __global__ void __launch_bounds__(256) reproject_kernel(
                 if (qx >= W || qx < 0 || qy >= H || qy < 0) continue;
                 // the reference reads prev_opacity here without the batch
                 // offset (ops/reproject.cu.cc:191)
-                if (__ldg(popac + (size_t)qy * W + qx) == 0.f) continue;
+                if (popac[(size_t)qy * W + qx] == 0.f) continue;
                 const size_t q = base + (size_t)qy * W + qx;
-                if (depth_normal_ok(Z, __ldg(plinz + 3 * q), fwZ, n, ld3(pnrm, q), fwN)) {
+                if (depth_normal_ok(Z, plinz[3 * q], fwZ, n, ld3(pnrm, q), fwN)) {
                     box |= 1u << k;
                     ++cnt;
                 }
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(256) reproject_kernel(
                 for (int s = 0; s < 4; ++s)
                     if (vmask & (1u << s)) {
                         const size_t q = base + (size_t)(ly + (s >> 1)) * W + (lx + (s & 1));
-                        acc = __fmaf_rn(w[s], __ldg(in + q * C + k), acc);
+                        acc = __fmaf_rn(w[s], in[q * C + k], acc);
                     }
                 acc = __fdiv_rn(acc, norm);
             } else if (mode == 2) {
@@ -191,7 +191,7 @@ __global__ void __launch_bounds__(256) reproject_kernel(
                 for (int s = 0; s < 9; ++s)
                     if (box & (1u << s)) {
                         const size_t q = base + (size_t)(ipy + s / 3 - 1) * W + (ipx + s % 3 - 1);
-                        acc = __fadd_rn(acc, __ldg(in + q * C + k));
+                        acc = __fadd_rn(acc, in[q * C + k]);
                     }
                 acc = __fdiv_rn(acc, norm);
             }
@@ -245,13 +245,13 @@ CD_DEV float bilinear(float ppx, float ppy, unsigned vmask, float w[4])
 // before; 48 registers (five blocks, its former occupancy), at the 56 it
 // would take 50.5.  The gather kernel keeps the chain: its sums need the
 // values too, and at five blocks with this form it took 63 us against 59.
-CD_DEV unsigned box_opacity(const float *__restrict__ popac, int ipx, int ipy, int W, int H)
+CD_DEV unsigned box_opacity(const float *popac, int ipx, int ipy, int W, int H)
 {
     float po[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         const int qx = ipx + (k % 3) - 1, qy = ipy + (k / 3) - 1;
-        po[k] = qx >= W || qx < 0 || qy >= H || qy < 0 ? 0.f : __ldg(popac + (size_t)qy * W + qx);
+        po[k] = qx >= W || qx < 0 || qy >= H || qy < 0 ? 0.f : popac[(size_t)qy * W + qx];
     }
     unsigned m = 0u;
 #pragma unroll
@@ -262,7 +262,7 @@ CD_DEV unsigned box_opacity(const float *__restrict__ popac, int ipx, int ipy, i
 
 // Of row j of that box, the taps among `open` (three bits) that pass the
 // depth and normal test.
-CD_DEV unsigned box_row(unsigned open, int j, const float *__restrict__ plinz, const float *__restrict__ pnrm,
+CD_DEV unsigned box_row(unsigned open, int j, const float *plinz, const float *pnrm,
                         size_t base, int ipx, int ipy, int W, float Z, float fwZ, float3 n, float fwN)
 {
     float zp[3];
@@ -271,7 +271,7 @@ CD_DEV unsigned box_row(unsigned open, int j, const float *__restrict__ plinz, c
     for (int i = 0; i < 3; ++i)
         if (open & (1u << i)) {
             const size_t q = base + (size_t)(ipy + j - 1) * W + (ipx + i - 1);
-            zp[i] = __ldg(plinz + 3 * q);
+            zp[i] = plinz[3 * q];
             np[i] = ld3(pnrm, q);
         }
     unsigned ok = 0u;
@@ -282,9 +282,9 @@ CD_DEV unsigned box_row(unsigned open, int j, const float *__restrict__ plinz, c
 }
 
 __global__ void __launch_bounds__(256, 5) reproject_decide_kernel(
-    const float *__restrict__ mvec, const float *__restrict__ linz, const float *__restrict__ plinz,
-    const float *__restrict__ nrm, const float *__restrict__ pnrm, const float *__restrict__ pnfw,
-    const float *__restrict__ opac, const float *__restrict__ popac, uint8_t *__restrict__ success, int H, int W)
+    const float *mvec, const float *linz, const float *plinz,
+    const float *nrm, const float *pnrm, const float *pnfw,
+    const float *opac, const float *popac, uint8_t *__restrict__ success, int H, int W)
 {
     chain_wait();
     chain_next();
@@ -294,9 +294,9 @@ __global__ void __launch_bounds__(256, 5) reproject_decide_kernel(
     const size_t base = (size_t)blockIdx.z * H * W;
     const size_t c = base + (size_t)cy * W + cx;
     uint8_t code = 0;
-    const float op = __ldg(opac + c), mx = __ldg(mvec + 3 * c), my = __ldg(mvec + 3 * c + 1);
-    const float fwN = __ldg(pnfw + 3 * c + 1);
-    const float Z = __ldg(linz + 3 * c), fwZ = __ldg(linz + 3 * c + 1);
+    const float op = opac[c], mx = mvec[3 * c], my = mvec[3 * c + 1];
+    const float fwN = pnfw[3 * c + 1];
+    const float Z = linz[3 * c], fwZ = linz[3 * c + 1];
     const float3 n = ld3(nrm, c);
     if (op != 0.f) {
         int ipx, ipy;
@@ -314,8 +314,8 @@ __global__ void __launch_bounds__(256, 5) reproject_decide_kernel(
                 po[s] = 0.f;
                 if (qx >= W || qx < 0 || qy >= H || qy < 0) continue;
                 const size_t q = base + (size_t)qy * W + qx;
-                po[s] = __ldg(popac + q);
-                zp[s] = __ldg(plinz + 3 * q);
+                po[s] = popac[q];
+                zp[s] = plinz[3 * q];
                 np[s] = ld3(pnrm, q);
             }
 #pragma unroll
@@ -335,10 +335,10 @@ __global__ void __launch_bounds__(256, 5) reproject_decide_kernel(
     success[c] = code;
 }
 
-__global__ void __launch_bounds__(256) reproject_gather_kernel(
-    const float *__restrict__ mvec, ReprojectList list, const float *__restrict__ linz,
-    const float *__restrict__ plinz, const float *__restrict__ nrm, const float *__restrict__ pnrm,
-    const float *__restrict__ pnfw, const float *__restrict__ popac, uint8_t *__restrict__ success, int H, int W)
+__global__ void __launch_bounds__(256, 5) reproject_gather_kernel(
+    const float *mvec, ReprojectList list, const float *linz,
+    const float *plinz, const float *nrm, const float *pnrm,
+    const float *pnfw, const float *popac, uint8_t *success, int H, int W)
 {
     chain_wait();
     chain_next();
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(256) reproject_gather_kernel(
     for (int d = 0; d < 3; ++d) acc[d][0] = acc[d][1] = acc[d][2] = 0.f;
     float norm = 1.f;
     if (code) {
-        const float mx = __ldg(mvec + 3 * c), my = __ldg(mvec + 3 * c + 1);
+        const float mx = mvec[3 * c], my = mvec[3 * c + 1];
         int ipx, ipy;
         float ppx, ppy;
         reproject_taps(mx, my, cx, cy, W, H, ipx, ipy, ppx, ppy);
@@ -381,16 +381,16 @@ __global__ void __launch_bounds__(256) reproject_gather_kernel(
                     }
         } else {
             // the 3x3 box, re-tested (the decision kernel keeps one bit)
-            const float fwN = __ldg(pnfw + 3 * c + 1);
-            const float Z = __ldg(linz + 3 * c), fwZ = __ldg(linz + 3 * c + 1);
+            const float fwN = pnfw[3 * c + 1];
+            const float Z = linz[3 * c], fwZ = linz[3 * c + 1];
             const float3 n = ld3(nrm, c);
             int cnt = 0;
             for (int k = 0; k < 9; ++k) {
                 const int qx = ipx + (k % 3) - 1, qy = ipy + (k / 3) - 1;
                 if (qx >= W || qx < 0 || qy >= H || qy < 0) continue;
-                if (__ldg(popac + (size_t)qy * W + qx) == 0.f) continue;
+                if (popac[(size_t)qy * W + qx] == 0.f) continue;
                 const size_t q = base + (size_t)qy * W + qx;
-                if (!depth_normal_ok(Z, __ldg(plinz + 3 * q), fwZ, n, ld3(pnrm, q), fwN)) continue;
+                if (!depth_normal_ok(Z, plinz[3 * q], fwZ, n, ld3(pnrm, q), fwN)) continue;
                 ++cnt;
 #pragma unroll
                 for (int d = 0; d < 3; ++d) {

@@ -28,10 +28,10 @@ namespace {
 using fsw::f2;
 
 template <int HW>
-__global__ void __launch_bounds__(256) sf_forward_kernel(
-    const float *__restrict__ imga, const float *__restrict__ imgb,
-    const float *__restrict__ albedo, const float *__restrict__ normal,
-    const float *__restrict__ band, float *__restrict__ acca, float *__restrict__ accb,
+__global__ void __launch_bounds__(256, 4) sf_forward_kernel(
+    const float *imga, const float *imgb,
+    const float *albedo, const float *normal,
+    const float *band, float *__restrict__ acca, float *__restrict__ accb,
     float *__restrict__ wsa, float *__restrict__ wsb, int H, int W, int hw_rt)
 {
     chain_wait();
@@ -62,11 +62,11 @@ __global__ void __launch_bounds__(256) sf_forward_kernel(
 // forward and gradient of a 719x1277 frame, window 11, 527 -> 519 us.
 template <int HW>
 __global__ void __launch_bounds__(256, 2) sf_grad_kernel(
-    const float *__restrict__ gacca, const float *__restrict__ gaccb,
-    const float *__restrict__ gwsa, const float *__restrict__ gwsb,
-    const float *__restrict__ imga, const float *__restrict__ imgb,
-    const float *__restrict__ albedo, const float *__restrict__ normal,
-    const float *__restrict__ band, float *__restrict__ gband, int H, int W, int hw_rt)
+    const float *gacca, const float *gaccb,
+    const float *gwsa, const float *gwsb,
+    const float *imga, const float *imgb,
+    const float *albedo, const float *normal,
+    const float *band, float *__restrict__ gband, int H, int W, int hw_rt)
 {
     chain_wait();
     chain_next();
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(256, 2) sf_grad_kernel(
     // accumulated in registers and dotted with the upstream gradient as
     // SpatialFilterGradKernel does (:64-80)
     fsw::sweep<HW, false, true>(tile, pdtab, hw, c, s);
-    fsw::band_grad(s, ld3(gacca, p), ld3(gaccb, p), __ldg(gwsa + p), __ldg(gwsb + p), gband + 5 * p);
+    fsw::band_grad(s, ld3(gacca, p), ld3(gaccb, p), gwsa[p], gwsb[p], gband + 5 * p);
 }
 
 // Stored-partials variant, the reference's design (its forward keeps 128 B
@@ -98,9 +98,9 @@ __global__ void __launch_bounds__(256, 2) sf_grad_kernel(
 // measurement; the sums are the recomputing kernels' to the bit.
 template <int HW>
 __global__ void __launch_bounds__(256) sf_forward_store_kernel(
-    const float *__restrict__ imga, const float *__restrict__ imgb,
-    const float *__restrict__ albedo, const float *__restrict__ normal,
-    const float *__restrict__ band, float *__restrict__ acca, float *__restrict__ accb,
+    const float *imga, const float *imgb,
+    const float *albedo, const float *normal,
+    const float *band, float *__restrict__ acca, float *__restrict__ accb,
     float *__restrict__ wsa, float *__restrict__ wsb, float4 *__restrict__ part, int H, int W, int hw_rt)
 {
     chain_wait();
@@ -131,11 +131,11 @@ __global__ void __launch_bounds__(256) sf_forward_store_kernel(
     }
 }
 
-__global__ void __launch_bounds__(256) sf_grad_stored_kernel(const float *__restrict__ gacca,
-                                                             const float *__restrict__ gaccb,
-                                                             const float *__restrict__ gwsa,
-                                                             const float *__restrict__ gwsb,
-                                                             const float4 *__restrict__ part,
+__global__ void __launch_bounds__(256) sf_grad_stored_kernel(const float *gacca,
+                                                             const float *gaccb,
+                                                             const float *gwsa,
+                                                             const float *gwsb,
+                                                             const float4 *part,
                                                              float *__restrict__ gband, size_t n)
 {
     chain_wait();
@@ -145,13 +145,13 @@ __global__ void __launch_bounds__(256) sf_grad_stored_kernel(const float *__rest
     fsw::Sums s;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float4 a = __ldg(part + 8 * p + k), bb = __ldg(part + 8 * p + 4 + k);
+        const float4 a = part[8 * p + k], bb = part[8 * p + 4 + k];
         s.px[k] = fsw::pack(a.x, bb.x);
         s.py[k] = fsw::pack(a.y, bb.y);
         s.pz[k] = fsw::pack(a.z, bb.z);
         s.pw[k] = fsw::pack(a.w, bb.w);
     }
-    fsw::band_grad(s, ld3(gacca, p), ld3(gaccb, p), __ldg(gwsa + p), __ldg(gwsb + p), gband + 5 * p);
+    fsw::band_grad(s, ld3(gacca, p), ld3(gaccb, p), gwsa[p], gwsb[p], gband + 5 * p);
 }
 
 template <typename F>

@@ -53,11 +53,11 @@ CD_DEV float eroded_at(const uint8_t *mask, int x, int y, int H, int W)
     float m = 1.f;
     for (int yy = max(0, y - 1); yy <= min(H - 1, y + 1); ++yy)
         for (int xx = max(0, x - 1); xx <= min(W - 1, x + 1); ++xx)
-            m = fminf(m, __ldg(mask + (size_t)yy * W + xx) ? 1.f : 0.f);
+            m = fminf(m, mask[(size_t)yy * W + xx] ? 1.f : 0.f);
     return m;
 }
 
-__global__ void __launch_bounds__(256) erode_kernel(const uint8_t *__restrict__ mask,
+__global__ void __launch_bounds__(256) erode_kernel(const uint8_t *mask,
                                                     float *__restrict__ out, int H, int W)
 {
     chain_wait();
@@ -71,10 +71,10 @@ __global__ void __launch_bounds__(256) erode_kernel(const uint8_t *__restrict__ 
 
 template <bool kFused>
 __global__ void __launch_bounds__(kTX * kTY, 3) temporal_kernel(
-    const float *__restrict__ cur1, const float *__restrict__ cur2,
-    const float *__restrict__ prev, const float *__restrict__ prev1,
-    const float *__restrict__ prev2, const float *__restrict__ rs,
-    const uint8_t *__restrict__ raw, float *__restrict__ eroded, float *__restrict__ out,
+    const float *cur1, const float *cur2,
+    const float *prev, const float *prev1,
+    const float *prev2, const float *rs,
+    const uint8_t *raw, float *__restrict__ eroded, float *__restrict__ out,
     float *__restrict__ out1, float *__restrict__ out2, float *__restrict__ succ, int H, int W,
     int hc, int hp)
 {
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kTX * kTY, 3) temporal_kernel(
     if (kFused) {
         for (int i = tid; i < mw * mh; i += kTX * kTY) {
             const int r = i / mw, q = i - r * mw, gx = mx0 + q, gy = my0 + r;
-            smask[i] = gx >= 0 && gx < W && gy >= 0 && gy < H ? (__ldg(raw + (size_t)gy * W + gx) ? 1 : 0) : 1;
+            smask[i] = gx >= 0 && gx < W && gy >= 0 && gy < H ? (raw[(size_t)gy * W + gx] ? 1 : 0) : 1;
         }
     }
     __syncthreads();
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kTX * kTY, 3) temporal_kernel(
                           r0[2 * mw + 2];
         return v ? 1.f : 0.f;
     };
-    const float m = inside ? (kFused ? eroded_s(cx, cy) : __ldg(rs + p)) : 0.f;
+    const float m = inside ? (kFused ? eroded_s(cx, cy) : rs[p]) : 0.f;
     // row pass: min/max along x over 2*hc+1 tile columns
     for (int t = tid; t < rplane; t += kTX * kTY) {
         const int r = t / kTX, x = t - r * kTX;
@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(kTX * kTY, 3) temporal_kernel(
             if (ix < 0 || ix >= W || iy < 0 || iy >= H) continue;
             const size_t q = (size_t)iy * W + ix;
             const bool centre = ix == cx && iy == cy;
-            const float mq = centre ? m : (kFused ? eroded_s(ix, iy) : __ldg(rs + q));
+            const float mq = centre ? m : (kFused ? eroded_s(ix, iy) : rs[q]);
             if (mq < 1.f) continue;
             const float3 v0 = centre ? h0 : ld3(prev, q), v1 = centre ? h1 : ld3(prev1, q);
             const float3 v2 = centre ? h2 : ld3(prev2, q);

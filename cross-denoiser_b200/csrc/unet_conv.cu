@@ -142,8 +142,8 @@ __device__ __forceinline__ void conv_out_row(const ConvParams &P, const float *v
                 lo += bias[j];
                 hi += bias[j + 1];
             } else if (P.bias) {
-                lo += __ldg(P.bias + j);
-                hi += __ldg(P.bias + j + 1);
+                lo += P.bias[j];
+                hi += P.bias[j + 1];
             }
             const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
             o[e] = *reinterpret_cast<const uint32_t *>(&h);
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
         const uint32_t lanes = tbase + ((uint32_t)((warp & 3) * 32) << 16);
         float bias[NOUT];
 #pragma unroll
-        for (int j = 0; j < NOUT; ++j) bias[j] = P.bias ? __ldg(P.bias + j) : 0.f;   // zeros: no bias
+        for (int j = 0; j < NOUT; ++j) bias[j] = P.bias ? P.bias[j] : 0.f;   // zeros: no bias
         for (int i = 0; i < ntile; ++i) {
             const int buf = i % kBufs, tile = first + i * stride;
             bool got = true;
@@ -662,7 +662,7 @@ bool pipe_steps_supported(int n) { return n == 2 || n == 3 || n == 5 || n == 6 |
 // conv input channel 8 * chunk + e to conv output channel n; in a ky-stacked
 // table the rows are 3 * nout, row n' holding tap ky = 2 - n' / nout of
 // output channel n' % nout.
-__device__ __forceinline__ void pack_one(const float *__restrict__ w, __nv_bfloat16 *__restrict__ dst,
+__device__ __forceinline__ void pack_one(const float *w, __nv_bfloat16 *__restrict__ dst,
                                          const PackTable &T, int i)
 {
     const int rows = T.stacked ? 3 * T.nout : T.nout;
@@ -687,7 +687,7 @@ __device__ __forceinline__ void pack_one(const float *__restrict__ w, __nv_bfloa
     dst[i] = __float2bfloat16_rn(v);
 }
 
-__global__ void pack_kernel(const float *__restrict__ w, __nv_bfloat16 *__restrict__ dst, const PackTable T)
+__global__ void pack_kernel(const float *w, __nv_bfloat16 *__restrict__ dst, const PackTable T)
 {
     chain_wait();
     chain_next();

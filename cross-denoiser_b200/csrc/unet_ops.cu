@@ -48,9 +48,9 @@ CD_DEV void st8(__nv_bfloat16 *p, const float *v) { *reinterpret_cast<uint4 *>(p
 
 // [ols1, ols2, prev_out, albedo, normal] (fp32, 3 channels each) -> bf16, 16
 // channels (15 + zero) in two row-chunk planes; n = B * H * W pixels, W wide
-__global__ void __launch_bounds__(256) pack_input_kernel(const float *__restrict__ a, const float *__restrict__ b,
-                                                         const float *__restrict__ c, const float *__restrict__ d,
-                                                         const float *__restrict__ e, __nv_bfloat16 *__restrict__ x,
+__global__ void __launch_bounds__(256) pack_input_kernel(const float *a, const float *b,
+                                                         const float *c, const float *d,
+                                                         const float *e, __nv_bfloat16 *__restrict__ x,
                                                          size_t n, int W)
 {
     chain_wait();
@@ -62,9 +62,9 @@ __global__ void __launch_bounds__(256) pack_input_kernel(const float *__restrict
     const float *src[5] = {a, b, c, d, e};
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
-        v[3 * k] = __ldg(src[k] + 3 * p);
-        v[3 * k + 1] = __ldg(src[k] + 3 * p + 1);
-        v[3 * k + 2] = __ldg(src[k] + 3 * p + 2);
+        v[3 * k] = src[k][3 * p];
+        v[3 * k + 1] = src[k][3 * p + 1];
+        v[3 * k + 2] = src[k][3 * p + 2];
     }
     v[15] = 0.f;
     st8(x + act_idx(0, row, 0, px, 0, W, 2) * 8, v);
@@ -80,8 +80,8 @@ __global__ void __launch_bounds__(256) pack_input_kernel(const float *__restrict
 // every store is 512 consecutive bytes: 32 channels at 480x270 22 -> 16 us, 16
 // at 960x540 27 -> 18.
 template <int CI, int CO, int kPix>
-__global__ void __launch_bounds__(256) tconv_fwd_kernel(const __nv_bfloat16 *__restrict__ in,
-                                                        const float *__restrict__ K, const float *__restrict__ bias,
+__global__ void __launch_bounds__(256) tconv_fwd_kernel(const __nv_bfloat16 *in,
+                                                        const float *K, const float *bias,
                                                         __nv_bfloat16 *__restrict__ out, int Hi, int Wi, int B)
 {
     chain_wait();
@@ -155,9 +155,9 @@ __global__ void __launch_bounds__(256) tconv_fwd_kernel(const __nv_bfloat16 *__r
 // of each input pixel).  Blocks walk chunks blockIdx.x, + gridDim.x, ...
 // and keep their dK / db sums in registers: one partial row per block.
 template <int CI, int CO, int kN>
-__global__ void __launch_bounds__(kN) tconv_bwd_kernel(const __nv_bfloat16 *__restrict__ in,
-                                                        const __nv_bfloat16 *__restrict__ dout,
-                                                        const float *__restrict__ K,
+__global__ void __launch_bounds__(kN) tconv_bwd_kernel(const __nv_bfloat16 *in,
+                                                        const __nv_bfloat16 *dout,
+                                                        const float *K,
                                                         __nv_bfloat16 *__restrict__ dz_in, float *__restrict__ partial,
                                                         int Hi, int Wi, int B)
 {
@@ -305,9 +305,9 @@ CD_DEV void head_params(const float4 *sT, const float *bias, const float (&v)[2]
     }
 }
 
-__global__ void __launch_bounds__(kHeadThreads) head_fwd_kernel(const __nv_bfloat16 *__restrict__ x,
-                                                                const float *__restrict__ K,
-                                                                const float *__restrict__ bias,
+__global__ void __launch_bounds__(kHeadThreads) head_fwd_kernel(const __nv_bfloat16 *x,
+                                                                const float *K,
+                                                                const float *bias,
                                                                 float *__restrict__ band, float *__restrict__ alpha,
                                                                 size_t n)
 {
@@ -374,11 +374,11 @@ CD_DEV void head_cp(void *dst, const void *src, int bytes)   // bytes: 4 or 16
     else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
-__global__ void __launch_bounds__(kHeadThreads, 2) head_bwd_kernel(const __nv_bfloat16 *__restrict__ x,
-                                                                   const float *__restrict__ K,
-                                                                   const float *__restrict__ bias,
-                                                                   const float *__restrict__ gband,
-                                                                   const float *__restrict__ galpha,
+__global__ void __launch_bounds__(kHeadThreads, 2) head_bwd_kernel(const __nv_bfloat16 *x,
+                                                                   const float *K,
+                                                                   const float *bias,
+                                                                   const float *gband,
+                                                                   const float *galpha,
                                                                    __nv_bfloat16 *__restrict__ dz,
                                                                    float *__restrict__ partial, size_t n)
 {
@@ -505,10 +505,10 @@ __global__ void __launch_bounds__(kHeadThreads, 2) head_bwd_kernel(const __nv_bf
 // pixels of its 2x2 window once per 8-channel chunk; the pooled gradient
 // goes to the first maximum of the window (row-major), as in the forward.
 template <int C>
-__global__ void __launch_bounds__(256) pool_bwd_kernel(const __nv_bfloat16 *__restrict__ act,
-                                                       const __nv_bfloat16 *__restrict__ pooled,
-                                                       const __nv_bfloat16 *__restrict__ dpool,
-                                                       const __nv_bfloat16 *__restrict__ dskip,
+__global__ void __launch_bounds__(256) pool_bwd_kernel(const __nv_bfloat16 *act,
+                                                       const __nv_bfloat16 *pooled,
+                                                       const __nv_bfloat16 *dpool,
+                                                       const __nv_bfloat16 *dskip,
                                                        __nv_bfloat16 *__restrict__ dz, int H, int W, int B)
 {
     chain_wait();
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(32 * kReduceWarps) reduce_kernel(const __grid_
     float s = 0.f;
     if (j < n) {
 #pragma unroll 4
-        for (int t = warp; t < rows; t += kReduceWarps) s += __ldg(partial + (size_t)t * n + j);
+        for (int t = warp; t < rows; t += kReduceWarps) s += partial[(size_t)t * n + j];
     }
     red[warp][lane] = s;
     __syncthreads();
@@ -586,9 +586,8 @@ __global__ void __launch_bounds__(32 * kReduceWarps) reduce_kernel(const __grid_
 // The update count lives in device memory (so a captured graph replays
 // correct steps): t = *step + 1, lr_t = lr sqrt(1 - b2^t) / (1 - b1^t) in
 // float as Keras computes it; step_kernel then advances the counter.
-__global__ void __launch_bounds__(256) adam_kernel(float *__restrict__ w, const float *__restrict__ g,
-                                                   float *__restrict__ m, float *__restrict__ v, int n,
-                                                   const int *__restrict__ step, float lr, float b1, float b2,
+__global__ void __launch_bounds__(256) adam_kernel(float *w, const float *g, float *m, float *v, int n,
+                                                   const int *step, float lr, float b1, float b2,
                                                    float eps)
 {
     chain_wait();
