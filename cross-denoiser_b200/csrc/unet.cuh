@@ -43,7 +43,7 @@ struct ConvParams {
     const __nv_bfloat16 *src0, *src1;   // inputs, c0 and c1 chunks per pixel (concatenated)
     int c0, c1;
     const __nv_bfloat16 *wpack;         // packed B operand, nsteps * 2 * NOUT * 8 bf16
-    const float *bias;                  // [NOUT] or null
+    const float *bias;                  // [8 (d0 + d1)] or null
     __nv_bfloat16 *dst0, *dst1;         // outputs, d0 and d1 chunks per pixel
     int d0, d1;
     const __nv_bfloat16 *mask0, *mask1; // ReLU masks laid out like dst0 / dst1, or null
@@ -54,6 +54,18 @@ struct ConvParams {
     int *err;                           // set to 1 if an MMA wait times out
     KStep steps[kMaxSteps];
 };
+
+// The bias of every output channel that is stored, zero for the padding up to
+// NOUT: a layer of 8 outputs has 8 of them in memory.
+template <int NOUT>
+__host__ __device__ inline void conv_bias(const ConvParams &P, float (&v)[NOUT])
+{
+    const int n = P.bias ? 8 * (P.d0 + P.d1) : 0;
+#ifdef __CUDA_ARCH__
+#pragma unroll
+#endif
+    for (int j = 0; j < NOUT; ++j) v[j] = j < n ? P.bias[j] : 0.f;
+}
 
 int build_steps(int c0, int c1, KStep *steps, StepHalf (*half)[2]);
 // The same taps as build_steps with the three vertical taps of each (kx,

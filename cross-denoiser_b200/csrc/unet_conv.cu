@@ -570,8 +570,7 @@ __global__ void __launch_bounds__(kPipeThreads, 2)
         const int m = (warp & 3) * 32 + lane, rp = ew >> 2;
         const uint32_t lanes = tbase + ((uint32_t)((warp & 3) * 32) << 16);
         float bias[NOUT];
-#pragma unroll
-        for (int j = 0; j < NOUT; ++j) bias[j] = P.bias ? P.bias[j] : 0.f;   // zeros: no bias
+        conv_bias<NOUT>(P, bias);
         for (int i = 0; i < ntile; ++i) {
             const int buf = i % kBufs, tile = first + i * stride;
             bool got = true;
