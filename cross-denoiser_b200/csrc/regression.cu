@@ -632,9 +632,22 @@ __global__ void __launch_bounds__(kThreads, 8) regression_kernel(
 constexpr int kRX = 32, kRThreadRows = 4;
 constexpr int kRec = 13;   // float4 per staged centre
 
-// Two pixels per thread while three CTAs' centres fit an SM's shared
-// memory, one for the wider windows and denser centres.
-constexpr size_t kReconPairSmem = 74 * 1024;
+// The three forms of the kernel and where each runs (us per cross-regression,
+// all with the same results):
+//   two pixels per thread (128 registers, four CTAs' worth) where a pixel
+//     reaches more than two centres a row, the grid still has two CTAs per SM
+//     of a 148-SM part, and three CTAs' centres fit an SM's shared memory.
+//     1080p, window 17, sparsity 4: 615 against 697 lean; 256x384 (384 CTAs),
+//     window 17: 72 against 75; below the lines: 192x192 (144 CTAs), window
+//     17: 65 against 64 lean, 64x96 64 against 62, 720p, window 5, sparsity 4:
+//     101 against 95, window 1, sparsity 2: 145 against 129;
+//   one, lean (72 registers, seven CTAs, the column loop not unrolled), while
+//     the centres of six CTAs fit: 720p, window 7, sparsity 4: 111 us, in the
+//     unrolled form of 111 registers 133;
+//   one, unrolled, for more centres than that, which leave few CTAs to an SM:
+//     720p, window 5, sparsity 1: 619 against 646 lean.
+constexpr size_t kReconPairSmem = 74 * 1024, kReconLeanSmem = 36 * 1024;
+constexpr long kReconPairCtas = 2 * 148;
 
 __host__ __device__ inline int floordiv(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
@@ -659,8 +672,8 @@ struct ReconPixel {
 // arithmetic); two pixels per thread read each record once for both.  The
 // rows of a warp's pixels are the same, so the centre rows that only one of
 // them reaches are a uniform branch.
-template <int NP>
-__global__ void __launch_bounds__(kRX * kRThreadRows, NP == 2 ? 4 : 1) recon_kernel(
+template <int NP, bool kLean>
+__global__ void __launch_bounds__(kRX * kRThreadRows, NP == 2 ? 4 : kLean ? 7 : 1) recon_kernel(
     const float *imga, const float *imgb,
     const float *albedo, const float *normal,
     const float *vara, const float *varb,
@@ -748,7 +761,7 @@ __global__ void __launch_bounds__(kRX * kRThreadRows, NP == 2 ? 4 : 1) recon_ker
     auto centre_row = [&](int iy, auto first, auto count) {
         constexpr int i0 = decltype(first)::value, n = decltype(count)::value;
         const float4 *R4 = rec + ((iy - cy_lo) * ncx - cx_lo + sx) * kRec;
-        for (int ix = sx; ix <= ex; ++ix, R4 += kRec) {
+        auto centre = [&]() {
             const ulonglong2 *R = reinterpret_cast<const ulonglong2 *>(R4);
             const ulonglong2 F9 = R[9], F10 = R[10], F11 = R[11];
             const float4 L12 = R4[12];
@@ -801,6 +814,12 @@ __global__ void __launch_bounds__(kRX * kRThreadRows, NP == 2 ? 4 : 1) recon_ker
                 q.o2 = fma2(w[i], p2, q.o2);
                 q.sw = add2(q.sw, w[i]);
             }
+        };
+        if (kLean) {
+#pragma unroll 1
+            for (int ix = sx; ix <= ex; ++ix, R4 += kRec) centre();
+        } else {
+            for (int ix = sx; ix <= ex; ++ix, R4 += kRec) centre();
         }
     };
     using std::integral_constant;
@@ -890,8 +909,12 @@ cudaError_t launch_recon(const float *imga, const float *imgb, const float *albe
         return launch_chained(kern, grid, block, smem, st, imga, imgb, albedo, normal, vara, varb, sda, sdb, beta,
                               outa, outb, state, H, W, hw, sp, rs);
     };
-    return recon_smem(hw, sp, rs, 2 * kRThreadRows) <= kReconPairSmem ? go(recon_kernel<2>, 2)
-                                                                      : go(recon_kernel<1>, 1);
+    constexpr int pair_rows = 2 * kRThreadRows;
+    const long pair_ctas = (long)B * ((Wr + kRX - 1) / kRX) * ((Hr + pair_rows - 1) / pair_rows);
+    if (win > 2 * sp && pair_ctas >= kReconPairCtas && recon_smem(hw, sp, rs, pair_rows) <= kReconPairSmem)
+        return go(recon_kernel<2, false>, 2);
+    return recon_smem(hw, sp, rs, kRThreadRows) <= kReconLeanSmem ? go(recon_kernel<1, true>, 1)
+                                                                  : go(recon_kernel<1, false>, 1);
 }
 
 }  // namespace cd
