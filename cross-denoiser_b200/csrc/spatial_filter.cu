@@ -57,11 +57,15 @@ __global__ void __launch_bounds__(256, 4) sf_forward_kernel(
     wsb[p] = fsw::hi(s.acc_w);
 }
 
-// Launch bound 2 CTAs per SM: the sweep is bound by the FMA pipe, and more
-// registers serve it better than a third CTA (80 registers and spills):
-// forward and gradient of a 719x1277 frame, window 11, 527 -> 519 us.
-template <int HW>
-__global__ void __launch_bounds__(256, 2) sf_grad_kernel(
+// kCtas, the launch bound in CTAs per SM.  From radius 3 on the sweep is bound
+// by the FMA pipe, and more registers serve it better than a third CTA (80
+// registers and spills): window 11 at 1920x1080 689 us with two, 706 with
+// three, window 9 496 and 513.  Below that staging the tile weighs more, and
+// in a grid that lasts the third CTA covers it: window 5 189 us against 197,
+// window 3 104 against 130, and 361x477 (690 CTAs), window 3, 10.5 against
+// 11.3, but window 5 19.5 against 19.0, and 64x96 4.2 against 3.9.
+template <int HW, int kCtas>
+__global__ void __launch_bounds__(256, kCtas) sf_grad_kernel(
     const float *gacca, const float *gaccb,
     const float *gwsa, const float *gwsb,
     const float *imga, const float *imgb,
@@ -223,14 +227,15 @@ cudaError_t launch_spatial_filter_grad(const float *gacca, const float *gaccb, c
     const int hw = win / 2;
     const size_t smem = fsw::smem_bytes(hw);
     dim3 grid((W + fsw::kBX - 1) / fsw::kBX, (H + fsw::kBY - 1) / fsw::kBY, B), block(fsw::kBX, fsw::kBY);
-    return dispatch_radius(hw, [&](auto r) {
-        constexpr int R = decltype(r)::value;
-        cudaError_t e = cudaFuncSetAttribute(sf_grad_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
+    auto go = [&](auto kern) {
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        return launch_chained(sf_grad_kernel<R>, grid, block, smem, st, gacca, gaccb, gwsa, gwsb, imga, imgb, albedo,
-                              normal, band, gband, H, W, hw);
-    });
+        return launch_chained(kern, grid, block, smem, st, gacca, gaccb, gwsa, gwsb, imga, imgb, albedo, normal, band,
+                              gband, H, W, hw);
+    };
+    const long ctas = (long)grid.x * grid.y * B;
+    if (hw < 3 && ctas > (hw < 2 ? 2 : 8) * 148) return go(sf_grad_kernel<0, 3>);
+    return dispatch_radius(hw, [&](auto r) { return go(sf_grad_kernel<decltype(r)::value, 2>); });
 }
 
 }  // namespace cd
