@@ -131,17 +131,6 @@ __device__ __forceinline__ void tmem_st16_zero(uint32_t taddr)
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// cp.async of 16 bytes with zero fill when src_bytes == 0.
-__device__ __forceinline__ void cp16(void *dst, const void *src, uint32_t src_bytes)
-{
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_wait_all()
-{
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-
 // ---------------------------------------------------------------------------
 // Bulk copies global -> shared, completing on an mbarrier whose transaction
 // count was raised with mbar_expect_tx.  Loads only, no multicast.

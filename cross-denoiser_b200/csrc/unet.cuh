@@ -112,7 +112,6 @@ struct WgradParams {
     int H, W;
     int *err;
 };
-size_t wgrad_tiles(int B, int H, int W);
 int wgrad_partial_rows(const WgradParams &P, int B);
 cudaError_t launch_wgrad(const WgradParams &P, int B, cudaStream_t st);
 

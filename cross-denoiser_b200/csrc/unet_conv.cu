@@ -702,127 +702,11 @@ __global__ void pack_jobs_kernel(const __grid_constant__ PackJobs J)
     pack_one(j.w, j.dst, j.T, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// Weight gradient.  D_tap[cin x cout] = sum_p X[p + tap][cin] dZ[p][cout]:
-// M = input channels (128 rows: the chunk planes of X from chunk 0 on), N =
-// output channels padded to NZ, K = 16 consecutive pixels per MMA; both
-// operands MN-major (channels contiguous, pixels 16 bytes apart).  Nine
-// accumulators, one per tap.  Each staged row carries, after its nch chunk
-// planes, a plane of ones, so row 8 * nch of the centre tap's accumulator is
-// sum_p dZ[p][cout], the bias gradient; rows past it read other staged data
-// and are discarded.  A CTA covers R rows x 128 pixels and writes its
-// partial sums [9 * cin * cout weights, cout biases].
-constexpr int kZPlane = kPx * 16;
-
-__host__ __device__ inline size_t wgrad_smem(int nch, int zc, int R)
-{
-    return (size_t)((R + 2) * (nch + 1) + 16) * kPlane + (size_t)(R * zc + 4) * kZPlane + 16;
-}
-
-template <int NZ, int R>
-__global__ void __launch_bounds__(128) wgrad_kernel(const WgradParams P)
-{
-    extern __shared__ __align__(128) uint8_t smem[];
-    constexpr int kCols = 9 * NZ <= 256 ? 256 : 512;
-    static_assert(9 * NZ <= 512, "nine accumulators of NZ columns");
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int x0 = blockIdx.x * kPx, y0 = blockIdx.y * R, b = blockIdx.z;
-    const int tile = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
-    const int nch = P.xc0 + P.xc1, rs = nch + 1;   // planes per staged row (with the ones plane)
-    uint8_t *sX = smem;
-    uint8_t *sZ = sX + (size_t)((R + 2) * rs + 16) * kPlane;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(sZ + (size_t)(R * P.zc + 4) * kZPlane);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 1);
-    for (int i = tid; i < (R + 2) * nch * kStagePx; i += 128) {
-        const int px = i % kStagePx, t = i / kStagePx;
-        const int c = t % nch, r = t / nch;
-        const int gy = y0 - 1 + r, gx = x0 - 1 + px;
-        const bool in = gy >= 0 && gy < P.H && gx >= 0 && gx < P.W;
-        const int yi = in ? gy : 0, xi = in ? gx : 0;
-        const __nv_bfloat16 *src = c < P.xc0 ? P.x0 + act_idx(b, yi, c, xi, P.H, P.W, P.xc0) * 8
-                                             : P.x1 + act_idx(b, yi, c - P.xc0, xi, P.H, P.W, P.xc1) * 8;
-        tc::cp16(sX + (size_t)(r * rs + c) * kPlane + 16 * px, src, in ? 16u : 0u);
-    }
-    const uint4 ones = make_uint4(0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u);   // bf16 1.0 x 8
-    for (int i = tid; i < (R + 2) * kStagePx; i += 128) {
-        const int px = i % kStagePx, r = i / kStagePx;
-        *reinterpret_cast<uint4 *>(sX + (size_t)(r * rs + nch) * kPlane + 16 * px) = ones;
-    }
-    for (int i = tid; i < R * P.zc * kPx; i += 128) {
-        const int px = i % kPx, t = i / kPx;
-        const int c = t % P.zc, r = t / P.zc;
-        const int gy = y0 + r, gx = x0 + px;
-        const bool in = gy < P.H && gx < P.W;
-        const __nv_bfloat16 *src = P.dz + act_idx(b, in ? gy : 0, c, in ? gx : 0, P.H, P.W, P.zc) * 8;
-        tc::cp16(sZ + (size_t)(r * P.zc + c) * kZPlane + 16 * px, src, in ? 16u : 0u);
-    }
-    if (warp == 0) tc::tmem_alloc(tslot, kCols);
-    if (tid == 0) tc::mbar_init(bar, 1);
-    tc::cp_wait_all();
-    tc::fence_async_smem();
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    const uint32_t tbase = *tslot;
-
-    if (tid == 0) {
-        const uint32_t idesc = tc::idesc_bf16(kPx, NZ) | (1u << 15) | (1u << 16);   // A and B MN-major
-        const uint32_t ax = tc::smem_u32(sX), az = tc::smem_u32(sZ);
-        for (int r = 0; r < R; ++r)
-            for (int g = 0; g < kPx / 16; ++g) {
-                const uint64_t bd = tc::sdesc(az + (uint32_t)(r * P.zc) * kZPlane + 256u * g, 128, kZPlane);
-                for (int tap = 0; tap < 9; ++tap) {
-                    const int ky = tap / 3, kx = tap - 3 * ky;
-                    const uint32_t a = ax + (uint32_t)((r + ky) * rs) * kPlane + (uint32_t)(kx + 16 * g) * 16;
-                    tc::mma_bf16(tbase + tap * NZ, tc::sdesc(a, 128, kPlane), bd, idesc, (r | g) ? 1u : 0u);
-                }
-            }
-        tc::commit(bar);
-    }
-    const bool done = __syncthreads_and(tc::mbar_wait(bar, 0, kWaitIter)) != 0;   // uniform across the CTA
-    tc::fence_after_sync();
-    float *out = P.partial + (size_t)tile * (9 * P.cin * P.cout + P.cout);
-    if (!done) {
-        if (tid == 0) atomicExch(P.err, 1);
-    } else if (warp * 32 <= 8 * nch) {
-        const int m = warp * 32 + (tid & 31);
-        for (int tap = 0; tap < 9; ++tap)
-#pragma unroll
-            for (int j = 0; j < NZ; j += 16) {
-                float v[16];
-                tc::tmem_ld16(tbase + ((uint32_t)(warp * 32) << 16) + tap * NZ + j, v);
-                if (m < P.cin) {
-#pragma unroll
-                    for (int q = 0; q < 16; ++q)
-                        if (j + q < P.cout) out[(tap * P.cin + m) * P.cout + j + q] = v[q];
-                } else if (m == 8 * nch && tap == 4) {
-#pragma unroll
-                    for (int q = 0; q < 16; ++q)
-                        if (j + q < P.cout) out[9 * P.cin * P.cout + j + q] = v[q];
-                }
-            }
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    if (warp == 0) tc::tmem_dealloc(tbase, kCols);
-}
+constexpr int kZPlane = kPx * 16;   // a staged row of one output-gradient chunk
 
 constexpr int kWgradLoadWarps = 2;
 constexpr int kWgradBiasWarps = 4;
 constexpr int kWgradThreads = 32 * (kWgradLoadWarps + 1 + kWgradBiasWarps);   // producers, MMA, bias
-
-constexpr int kWgradRows = 4;
-
-template <int NZ>
-cudaError_t launch_wgrad_t(const WgradParams &P, int B, cudaStream_t st)
-{
-    const size_t smem = smem_for_tmem(wgrad_smem(P.xc0 + P.xc1, P.zc, kWgradRows), 9 * NZ <= 256 ? 256 : 512);
-    cudaError_t e = cudaFuncSetAttribute(wgrad_kernel<NZ, kWgradRows>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    dim3 grid((P.W + kPx - 1) / kPx, (P.H + kWgradRows - 1) / kWgradRows, B);
-    wgrad_kernel<NZ, kWgradRows><<<grid, 128, smem, st>>>(P);
-    return cudaGetLastError();
-}
 
 // Persistent weight gradient of a 3x3 layer, two forms.
 //
@@ -1260,10 +1144,8 @@ cudaError_t launch_conv3x3(const ConvParams &P, int B, int nout, cudaStream_t st
             const ConvPipePlan p1 = conv_pipe_plan(P.nsteps, 3 * 16, P.c0, P.c1, Rs, kPipeSmem);
             if (p1.S >= 2) return launch_pipe<16, Rs>(P, p1, 1, B, st);
         }
-        if (nout == 16) return launch_t<16, kConvRowsStacked, true>(P, B, st);
-        if (nout == 32) return launch_t<32, kConvRowsStacked, true>(P, B, st);
-        if (nout == 48) return launch_t<48, kConvRowsStacked, true>(P, B, st);
-        return cudaErrorInvalidValue;
+        // 16 outputs only: the callers pack 32 and 48 for the per-row form
+        return nout == 16 ? launch_t<16, kConvRowsStacked, true>(P, B, st) : cudaErrorInvalidValue;
     }
     if (nout == 16) return launch_t<16, kConvRows, false>(P, B, st);
     if (nout == 32) return launch_rows<32, kConvRows>(P, B, st);
@@ -1294,16 +1176,13 @@ cudaError_t launch_pack(const float *w, __nv_bfloat16 *dst, const PackTable &T, 
     return launch_chained(pack_kernel, (n + 255) / 256, 256, 0, st, w, dst, T);
 }
 
-size_t wgrad_tiles(int B, int H, int W) { return (size_t)B * ((W + kPx - 1) / kPx) * ((H + kWgradRows - 1) / kWgradRows); }
-
-
 // CTAs of a layer's weight gradient: one per SM of a 148-SM part (a constant,
 // so that neither the workspace's size nor the sums' order depend on the
 // device).
 constexpr int kWgradCtas = 148;
 
-// The persistent kernel takes every layer whose (ky, cout) fit N
-// (zc <= 4) and whose input channels fit M (at most 16 chunks).  The
+// The kernel takes layers whose (ky, cout) fit N (zc <= 4) and whose input
+// channels fit M (at most 16 chunks): all that the entry points accept.  The
 // nine-tap form runs layers of one output-gradient chunk (N = 80 against
 // three MMAs of N = 32: 60 against 89 us at 1920x1080); at two chunks its
 // N = 144 MMAs measured slower than three of N = 48 (44 against 34 us at
@@ -1318,11 +1197,9 @@ static bool wgrad3_fits(const WgradParams &P)
     return P.zc >= 1 && P.zc <= 4 && xc >= 1 && xc <= 16 && wgrad3_plan_of(P).S >= 2;
 }
 
-// Partial-sum rows the weight gradient of this layer writes: one per CTA of
-// the persistent kernel, one per tile otherwise.
+// Partial-sum rows the weight gradient of this layer writes: one per CTA.
 int wgrad_partial_rows(const WgradParams &P, int B)
 {
-    if (!wgrad3_fits(P)) return (int)wgrad_tiles(B, P.H, P.W);
     const Wgrad3Plan p = wgrad3_plan_of(P);
     const int tiles = B * ((P.W + kPx - 1) / kPx) * ((P.H + p.R - 1) / p.R);
     return tiles < kWgradCtas ? tiles : kWgradCtas;
@@ -1330,18 +1207,15 @@ int wgrad_partial_rows(const WgradParams &P, int B)
 
 cudaError_t launch_wgrad(const WgradParams &P, int B, cudaStream_t st)
 {
-    if (P.cout > 32) return cudaErrorInvalidValue;
-    if (wgrad3_fits(P)) {
-        const int grid = wgrad_partial_rows(P, B);
-        const Wgrad3Plan p = wgrad3_plan_of(P);
-        switch (P.zc) {
-        case 1: return launch_wgrad3_t<1, true>(P, p, B, grid, st);
-        case 2: return launch_wgrad3_t<2, false>(P, p, B, grid, st);
-        case 3: return launch_wgrad3_t<3, false>(P, p, B, grid, st);
-        default: return launch_wgrad3_t<4, false>(P, p, B, grid, st);
-        }
+    if (!wgrad3_fits(P)) return cudaErrorInvalidValue;
+    const int grid = wgrad_partial_rows(P, B);
+    const Wgrad3Plan p = wgrad3_plan_of(P);
+    switch (P.zc) {
+    case 1: return launch_wgrad3_t<1, true>(P, p, B, grid, st);
+    case 2: return launch_wgrad3_t<2, false>(P, p, B, grid, st);
+    case 4: return launch_wgrad3_t<4, false>(P, p, B, grid, st);
+    default: return cudaErrorInvalidValue;
     }
-    return P.cout <= 16 ? launch_wgrad_t<16>(P, B, st) : launch_wgrad_t<32>(P, B, st);
 }
 
 }  // namespace unet
