@@ -211,9 +211,16 @@ CD_DEV float exp_ftz(float x)
 // functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34,
 // 1990): with y the reciprocal of b rounded to nearest, q = RN(a y) and the
 // exact residual r = a - q b, RN(q + r y) is the IEEE quotient a / b.  y is
-// the hardware approximation (1 ulp) after one Newton step, which differs
-// from the rounded reciprocal only within about 2^-46 of a rounding
-// boundary.  Valid while a, b, y and a / b stay away from the range's ends.
+// the hardware approximation after one Newton step: the rounded reciprocal
+// of every significand (run on sm_100a over all 2^23 of them at nine
+// exponents; 7e10 quotients there equal the division's).
+// Holds for b in [2^-14, 2^100) and a = 0 or |a| in [2^-102, 2^100) with a
+// normal quotient.  Below, the residual (a multiple of 2^-47 of a) underflows
+// and the result may be an ulp off.  That is not seen: with the taps' divisors
+// of 1e-2 and more it is a difference quotient below 2^-95, whose square
+// vanishes beside the ridge of 1e-3 on the diagonal, and whose coefficient
+// multiplies a quotient as small in the reconstruction; a distance below
+// 2^-88 leaves its weight at 1.
 CD_DEV float reciprocal(float b)
 {
     float y;
@@ -251,18 +258,18 @@ struct Centre {
 // Follows ops/regression.cu.cc:418-445: delta = [1, (f_t-f_c)/(sd_c+sd_t+1e-2),
 // alb_t-alb_c, n_t-n_c], w = exp(-|f_t-f_c|^2/(v_c+v_t+1e-4)) + 1e-7.
 //
-// The tap's four quotients are the IEEE quotients: the normal equations
-// amplify their last bits.  kFast takes them with quotient() from two
-// reciprocals instead of four divisions (about 20 instructions each, with a
-// branch): 1080p, window 17, the kernel 505 -> 433 us (and 407 us with the
-// pairs, the fixed row layout and the launch bound below).  That needs the
-// divisors (at least 1e-4) and the squared distance below kQuotientMax,
-// which bounds the other operands too (sd = sqrt(v)); `sane` turns false
-// where a tap is not, and the caller starts its window again with kFast off
-// at the end of that row.  256x256, window 15, one NaN pixel: 125 us (151 with
-// four divisions throughout, 197 when the window was swept to its end and
-// repeated with them); 1080p, window 17, 3000 of them: 952 (1110, 1406).
-// The vote per row costs a finite frame 0.5 %.
+// The tap's four quotients are the IEEE quotients (but for the smallest, see
+// quotient()): the normal equations amplify their last bits.  kFast takes them
+// with quotient() from two reciprocals instead of four divisions (about 20
+// instructions each, with a branch): 1080p, window 17, the kernel 505 -> 433
+// us (and 407 us with the pairs, the fixed row layout and the launch bound
+// below).  That needs the divisors (at least 1e-4) and the squared distance
+// below kQuotientMax, which bounds the other operands from above too (sd =
+// sqrt(v)); `sane` turns false where a tap is not, and the caller starts its
+// window again with kFast off at the end of that row.  256x256, window 15, one
+// NaN pixel: 125 us (151 with four divisions throughout, 197 when the window
+// was swept to its end and repeated with them); 1080p, window 17, 3000 of
+// them: 952 (1110, 1406).  The vote per row costs a finite frame 0.5 %.
 template <bool kFast>
 CD_DEV void normal_tap(Normal &n, float4 f4, float4 y4, float4 a4, float4 n4, float sdt, const Centre &c, bool &sane)
 {
