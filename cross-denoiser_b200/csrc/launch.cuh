@@ -16,11 +16,14 @@
 //   * chain_next() lets the next kernel's CTAs start; a kernel that allocates
 //     TMEM does so after chain_wait() and calls chain_next() after the
 //     allocation, so no waiting CTA ever holds TMEM that an earlier kernel's
-//     CTA still has to allocate.
+//     CTA still has to allocate.  Where a grid is about one wave it is left
+//     out: the next kernel's CTAs then start as this one's end, not in the
+//     slots that the wave leaves free (temporal.cu).
 // A kernel launched any other way after one of these starts when it has
-// ended, as always.  On the U-Net's 12 forward and 16 chained backward
-// kernels: prediction at 1920x1080 315 -> 295 us, a training pass at
-// 2560x1440 1498 -> 1447 us, a whole 256x256 training step 455 -> 427 us.
+// ended, as always.  On the U-Net's 14 forward and 15 chained backward
+// kernels (the nine weight gradients are launched plainly): prediction at
+// 1920x1080 315 -> 295 us, a training pass at 2560x1440 1498 -> 1447 us, a
+// whole 256x256 training step 455 -> 427 us.
 #pragma once
 #include <utility>
 #include <cuda_runtime.h>

@@ -892,7 +892,8 @@ cudaError_t launch_regression(const float *imga, const float *imgb, const float 
         const size_t smem = regression_smem(g);
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
-        kern<<<grid, kThreads, smem, st>>>(imga, imgb, albedo, normal, vara, varb, sda, sdb, beta, chol, cond_limit, fallbacks, H, W, hw, sp);
+        kern<<<grid, kThreads, smem, st>>>(imga, imgb, albedo, normal, vara, varb, sda, sdb, beta, chol, cond_limit,
+                                           fallbacks, H, W, hw, sp);
         return cudaGetLastError();
     };
     if (!fixed_rows(hw, sp)) return go(regression_kernel<0>, regression_geom<0>(hw, sp));
